@@ -473,6 +473,14 @@ LOC_API long loc_write_positions_text(const double *rows, const uint8_t *flags, 
 LOC_API long loc_find_candidates(const uint16_t *d_frames, int n_frames, int n_rows, int n_cols, double pfa,
                                  double psf_width, loc_candidate *d_cands, long max_cands, void *stream);
 
+/* The same search where the caller does not know how many candidates there
+ * are: once they are counted, alloc(user, n) is called once on the calling
+ * thread (not at all if n is 0) and returns device memory for n candidates,
+ * which receives them all. Returns n. */
+typedef void *(*loc_alloc_fn)(void *user, long n);
+LOC_API long loc_find_candidates_alloc(const uint16_t *d_frames, int n_frames, int n_rows, int n_cols, double pfa,
+                                       double psf_width, loc_alloc_fn alloc, void *user, void *stream);
+
 /*
  * Learned start proposal (no reference counterpart: the reference starts
  * every fit from the finder's centroid and the PSF width, Localization.cpp

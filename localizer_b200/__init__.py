@@ -85,6 +85,8 @@ class Tuning(C.Structure):
         return {n: (float(getattr(self, n)) if n.startswith("ms_") else int(getattr(self, n))) for n, _ in self._fields_}
 
 
+_AllocFn = C.CFUNCTYPE(C.c_void_p, C.c_void_p, C.c_long)   # loc_alloc_fn
+
 # names and prototypes of every exported entry point of include/localizer_b200.h
 _PROTOS = {
     "loc_default_options": (None, [C.POINTER(Options)]),
@@ -122,6 +124,8 @@ _PROTOS = {
     "loc_write_positions_text": (C.c_long, [C.c_void_p, C.c_void_p, C.c_long, C.c_int, C.c_char_p, C.c_char_p]),
     "loc_find_candidates": (C.c_long, [C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_double, C.c_double, C.c_void_p,
                                        C.c_long, C.c_void_p]),
+    "loc_find_candidates_alloc": (C.c_long, [C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_double, C.c_double, _AllocFn,
+                                             C.c_void_p, C.c_void_p]),
     "loc_proposal_weight_count": (C.c_int, [C.c_int]),
     "loc_proposal_create": (C.c_int, [C.POINTER(C.c_void_p), C.c_int, C.c_int, C.c_ulonglong]),
     "loc_proposal_destroy": (C.c_int, [C.c_void_p]),
@@ -341,14 +345,22 @@ def find_candidates_device(frames, pfa: float, psf_width: float, stream: int = 0
     find_candidates on the same frames."""
     import torch
     n_frames, n_cols, n_rows = frames.shape
-    cap = max(1024, n_frames * 64)
-    while True:
-        out = torch.empty(cap * CANDIDATE_DTYPE.itemsize, dtype=torch.uint8, device=frames.device)
-        n = _check(lib().loc_find_candidates(C.c_void_p(frames.data_ptr()), n_frames, n_rows, n_cols, pfa,
-                                             psf_width, C.c_void_p(out.data_ptr()), cap, C.c_void_p(stream)))
-        if n <= cap:
-            return out[:n * CANDIDATE_DTYPE.itemsize], n
-        cap = n
+    found, failed = [], []
+
+    def alloc(_, n):
+        try:
+            found.append(torch.empty(n * CANDIDATE_DTYPE.itemsize, dtype=torch.uint8, device=frames.device))
+        except Exception as e:   # out of memory: raised below, not inside the C call
+            failed.append(e)
+            return None
+        return found[0].data_ptr()
+
+    n = lib().loc_find_candidates_alloc(C.c_void_p(frames.data_ptr()), n_frames, n_rows, n_cols, pfa, psf_width,
+                                        _AllocFn(alloc), None, C.c_void_p(stream))
+    if failed:
+        raise failed[0]
+    _check(n)
+    return (found[0] if found else torch.empty(0, dtype=torch.uint8, device=frames.device)), n
 
 
 STORAGE_FORMATS = {"int8": 2, "uint8": 3, "int16": 4, "uint16": 5, "int32": 6, "uint32": 7, "int64": 8,

@@ -64,8 +64,7 @@ def test_hard_statistics():
 
 def test_many_runs():
     """Noise at a low threshold: more runs per frame than the shared table,
-    more particles than the first guess of the particle table; several
-    threads' worth of frames in one call."""
+    more particles than the first guess of the particle table."""
     rng = np.random.default_rng(9)
     frames = rng.poisson(100, size=(3, 400, 420)).astype(np.uint16)
     assert _check(frames, 2.0, 0.7) > 4000
