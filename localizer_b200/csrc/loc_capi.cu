@@ -332,9 +332,6 @@ struct loc_ctx {
     cudaStream_t aux[locb::kMaxAux] = {};
     cudaEvent_t fork = nullptr;
     cudaEvent_t join[locb::kMaxAux] = {};
-    cudaStream_t aux_long[locb::kMaxAux] = {};
-    cudaEvent_t flagged[locb::kMaxAux] = {};
-    cudaEvent_t join_long[locb::kMaxAux] = {};
     // launch shapes picked by loc_autotune, per method code; applied where
     // a call leaves the corresponding option at 0
     struct Shape {
@@ -413,10 +410,7 @@ LOC_API int loc_ctx_create(loc_ctx **ctx, int device)
         return cuda_fail(e, "cudaEventCreate");
     for (int k = 0; k < locb::kMaxAux; ++k) {
         if ((e = cudaStreamCreateWithFlags(&c->aux[k], cudaStreamNonBlocking)) != cudaSuccess ||
-            (e = cudaEventCreateWithFlags(&c->join[k], cudaEventDisableTiming)) != cudaSuccess ||
-            (e = cudaStreamCreateWithFlags(&c->aux_long[k], cudaStreamNonBlocking)) != cudaSuccess ||
-            (e = cudaEventCreateWithFlags(&c->flagged[k], cudaEventDisableTiming)) != cudaSuccess ||
-            (e = cudaEventCreateWithFlags(&c->join_long[k], cudaEventDisableTiming)) != cudaSuccess)
+            (e = cudaEventCreateWithFlags(&c->join[k], cudaEventDisableTiming)) != cudaSuccess)
             return cuda_fail(e, "auxiliary stream");
     }
     *ctx = c;
@@ -440,9 +434,6 @@ LOC_API int loc_ctx_destroy(loc_ctx *ctx)
     for (int k = 0; k < locb::kMaxAux; ++k) {
         if (ctx->aux[k]) cudaStreamDestroy(ctx->aux[k]);
         if (ctx->join[k]) cudaEventDestroy(ctx->join[k]);
-        if (ctx->aux_long[k]) cudaStreamDestroy(ctx->aux_long[k]);
-        if (ctx->flagged[k]) cudaEventDestroy(ctx->flagged[k]);
-        if (ctx->join_long[k]) cudaEventDestroy(ctx->join_long[k]);
     }
     for (cudaStream_t s : {ctx->s_in, ctx->s_fit, ctx->s_out})
         if (s) {
@@ -597,9 +588,6 @@ int fit_impl(loc_ctx *ctx, const uint16_t *d_frames, int n_frames, int n_rows, i
     for (int k = 0; k < locb::kMaxAux; ++k) {
         p.aux[k] = o.serial_classes ? nullptr : ctx->aux[k];
         p.join[k] = ctx->join[k];
-        p.aux_long[k] = o.serial_classes ? nullptr : ctx->aux_long[k];
-        p.flagged[k] = ctx->flagged[k];
-        p.join_long[k] = ctx->join_long[k];
     }
     p.fork = ctx->fork;
     p.out = d_out;

@@ -110,8 +110,8 @@ __device__ __forceinline__ float fsqrt(float a) { return a > 0.0f ? a * rsqrtf(a
 __device__ __forceinline__ double fsqrt(double a) { return sqrt(a); }
 
 // Per-fit array in registers, or (InSmem) in a shared-memory slot of the
-// fit's group; the FP64 solver keeps its normal equations, state vectors and
-// Cholesky factor there so that they are not live in registers.
+// fit's group; the FP64 thread groups keep their normal equations, state
+// vectors and Cholesky factor there so that they are not live in registers.
 template <typename T, int N, bool InSmem> struct StateArr;
 template <typename T, int N> struct StateArr<T, N, false> {
     T r[N];
@@ -125,6 +125,25 @@ template <typename T, int N> struct StateArr<T, N, true> {
     __device__ __forceinline__ T &operator[](int k) { return p[k]; }
     __device__ __forceinline__ const T &operator[](int k) const { return p[k]; }
 };
+
+// products that must round on their own, whatever they feed
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+
+// sum += x^2 for the terms i = 0, 1, ... (x0: the first): FP32 fuses every
+// term with the sum before it; FP64 fuses the first term with the rounded
+// second, then goes on the same way.
+template <typename T> __device__ __forceinline__ void add_square(T x, int i, T &x0, T &sum)
+{
+    if (i == 0) {
+        x0 = x;
+        sum = mul_rn(x, x);
+    } else if (i == 1 && sizeof(T) == 8) {
+        sum = fma(x0, x0, mul_rn(x, x));
+    } else {
+        sum = fma(x, x, sum);
+    }
+}
 
 template <typename T> __device__ __forceinline__ T tiny_pos();
 template <> __device__ __forceinline__ float tiny_pos<float>() { return FLT_MIN; }
@@ -175,6 +194,20 @@ __device__ __forceinline__ T expm1_series(T y)
     p = fma(y, p, T(0.5));
     p = fma(y, p, T(1));
     return y * p;
+}
+
+// Which product of the row term -dxs^2 - dys (2 w + dys) of pass_sym and
+// pass_fixed is fused with the other, rounded one: the square (true) or the
+// second. They differ in the last bit; each ROI side and group size has always
+// had the one given here, and every solver of a fit has to use it.
+template <typename T> __host__ __device__ constexpr bool row_fuse_square(int side, int threads)
+{
+    return threads > 1 && (sizeof(T) == 8 || side < 9 || side > 17);
+}
+template <typename T> __device__ __forceinline__ T row_term(int side, int threads, T dxs, T dys, T wy)
+{
+    const T t2 = fma(T(2), wy, dys);
+    return row_fuse_square<T>(side, threads) ? fma(-dxs, dxs, -mul_rn(dys, t2)) : fma(-dys, t2, -mul_rn(dxs, dxs));
 }
 
 // S > 0: compile-time ROI side (rows fully unrolled); S == 0: runtime side s_rt.
@@ -242,7 +275,7 @@ __device__ __forceinline__ void pass_sym(const float *__restrict__ roi, int ld, 
     for (int j = 0; j < s; ++j) {
         const T wy = (T)j - y0;
         const T wy2 = wy * wy;
-        const T krow = -dxs * dxs - dys * (T(2) * wy + dys);  // (d2' - d2) minus its u term
+        const T krow = S > 0 || TPF > 8 ? -dxs * dxs - dys * (T(2) * wy + dys) : row_term<T>(s, TPF, dxs, dys, wy);  // (d2' - d2) minus its u term
         const float *row = roi + j * s * ld;
         if (S > 0) {
             // two columns per trip: unrolling all of them made the per-class
@@ -311,7 +344,7 @@ __device__ __forceinline__ void pass_fixed(const float *__restrict__ roi, int ld
     for (int j = 0; j < s; ++j) {
         const T wy = (T)j - y0;
         const T wy2 = wy * wy;
-        const T krow = -dxs * dxs - dys * (T(2) * wy + dys);
+        const T krow = S > 0 || TPF > 8 ? -dxs * dxs - dys * (T(2) * wy + dys) : row_term<T>(s, TPF, dxs, dys, wy);
         const float *row = roi + j * s * ld;
         if (S > 0) {
             // two columns per trip: unrolling all of them made the per-class
@@ -448,6 +481,18 @@ __device__ __forceinline__ void pass_ell(const float *__restrict__ roi, int ld, 
     }
 }
 
+// Which of two roundings the FP32 symmetric solve uses in its forward
+// substitution, by ROI side and threads per fit: bit 0 for the undamped
+// solve, bit 1 for the damped ones. The two differ in the last bit of the
+// step; a size has always had the one given here, and every solver of a fit
+// has to use it for the fit's path to be the same in all of them.
+__host__ __device__ constexpr int sym_fuse(int side, int threads)
+{
+    return threads == 1 ? (side == 5 ? 0 : 3)
+         : threads != 8 ? 0
+         : (side >= 9 && side <= 13) || side == 7 || side == 5 ? 0 : 3;
+}
+
 // ---------------------------------------------------------------------------
 // Damped solve in D-scaled coordinates. With M = D^-1 J^T J D^-1 and
 // g = D^-1 J^T f, the lmpar step x (J x ~ f, reference step dx = -x) is
@@ -457,17 +502,20 @@ __device__ __forceinline__ void pass_ell(const float *__restrict__ roi, int ld, 
 // Result codes: 0 ok, 1 an FP32 pivot fell below thr * diagonal (redo in
 // FP64), 2 not positive definite (in the precision T).
 // ---------------------------------------------------------------------------
+// g = v invD. With fuse (some FP32 symmetric solves, see sym_fuse) the first
+// subtraction of the forward substitution takes the unrounded product (one
+// fused operation), else the rounded g.
+//
 // The triangular loops run over 0..P-1 with the bound as a condition
 // (same operations, same order): with trip counts that depend on the outer
 // index the compiler kept the factor and solve vectors in local memory for
 // P = 7.
-template <int P, typename T, typename MS, typename MA>
-__device__ __forceinline__ int chol_solve(const MA &Ms, MS par, const MS (&g)[P], T thr,
+template <int P, typename T, typename MS, bool LSM, typename MA>
+__device__ __forceinline__ int chol_solve(const MA &Ms, MS par, const MS (&v)[P], const MS (&invD)[P], bool fuse, T thr,
                                           MS (&z)[P], MS &znorm, MS &w2, MS &minpiv, T *lslot = nullptr)
 {
-    // the all-FP64 solve keeps its factor in the fit's shared-memory slot
-    constexpr bool kSm = sizeof(T) == 8 && sizeof(MS) == 8;
-    StateArr<T, tri(P), kSm> L(lslot);
+    constexpr bool kFuse = P == 5 && sizeof(T) == 4 && sizeof(MS) == 4;
+    StateArr<T, tri(P), LSM> L(lslot);   // LSM: the factor in the fit's shared-memory slot
     T inv[P];
     // smallest pivot ratio d / djj, kept as a fraction (one division at the
     // end instead of one per pivot: FP64 division is long-latency)
@@ -504,11 +552,16 @@ __device__ __forceinline__ int chol_solve(const MA &Ms, MS par, const MS (&g)[P]
     T y[P];
 #pragma unroll
     for (int i = 0; i < P; ++i) {
-        T sacc = (T)g[i];
+        T sacc;
+        sacc = (T)mul_rn(v[i], invD[i]);
+        if (i > 0) {
+            const T first = fma(-L[pkl(i, 0)], y[0], sacc);
+            sacc = kFuse && fuse ? fma((T)v[i], (T)invD[i], -mul_rn(L[pkl(i, 0)], y[0])) : first;
+        }
 #pragma unroll
-        for (int k = 0; k < P; ++k)
-            if (k < i) sacc -= L[pkl(i, k)] * y[k];
-        y[i] = sacc * inv[i];
+        for (int k = 1; k < P; ++k)
+            if (k < i) sacc = fma(-L[pkl(i, k)], y[k], sacc);
+        y[i] = mul_rn(sacc, inv[i]);
     }
     T zz[P];
 #pragma unroll
@@ -529,12 +582,13 @@ __device__ __forceinline__ int chol_solve(const MA &Ms, MS par, const MS (&g)[P]
         T qv[P];
 #pragma unroll
         for (int i = 0; i < P; ++i) {
-            T sacc = zz[i] * izn;
+            T sacc = mul_rn(zz[i], izn);
+            if (i > 0) sacc = fma(zz[i], izn, -mul_rn(L[pkl(i, 0)], qv[0]));
 #pragma unroll
-            for (int k = 0; k < P; ++k)
-                if (k < i) sacc -= L[pkl(i, k)] * qv[k];
-            qv[i] = sacc * inv[i];
-            q2 += qv[i] * qv[i];
+            for (int k = 1; k < P; ++k)
+                if (k < i) sacc = fma(-L[pkl(i, k)], qv[k], sacc);
+            qv[i] = mul_rn(sacc, inv[i]);
+            add_square<T>(qv[i], i, qv[0], q2);
         }
     }
 #pragma unroll
@@ -548,15 +602,19 @@ __device__ __forceinline__ int chol_solve(const MA &Ms, MS par, const MS (&g)[P]
 // Kept out of line: it is rare, and inlined its double-precision working set
 // would raise the register budget of the whole solver loop.
 template <int P>
-__device__ __noinline__ int chol_solve_fp64(const float *Ms, float par, const float *g, float *z, float *out)
+__device__ __noinline__ int chol_solve_fp64(const float *Ms, float par, const float *v, const float *invD, float *z,
+                                            float *out)
 {
-    float msl[tri(P)], gl[P], zl[P];
+    float msl[tri(P)], vl[P], dl[P], zl[P];
 #pragma unroll
     for (int k = 0; k < tri(P); ++k) msl[k] = Ms[k];
 #pragma unroll
-    for (int k = 0; k < P; ++k) gl[k] = g[k];
+    for (int k = 0; k < P; ++k) {
+        vl[k] = v[k];
+        dl[k] = invD[k];
+    }
     float zn, w2, mp;
-    const int rc = chol_solve<P, double, float>(msl, par, gl, 0.0, zl, zn, w2, mp);
+    const int rc = chol_solve<P, double, float, false>(msl, par, vl, dl, false, 0.0, zl, zn, w2, mp);
 #pragma unroll
     for (int k = 0; k < P; ++k) z[k] = zl[k];
     out[0] = zn;
@@ -568,24 +626,27 @@ __device__ __noinline__ int chol_solve_fp64(const float *Ms, float par, const fl
 // below thr * diagonal are refactorised in FP64. ESC is a separate kernel
 // instantiation: the out-of-line FP64 call costs the solver loop a stack
 // frame and register spills even when it never runs.
-template <int P, typename T, bool ESC, typename MA>
-__device__ __forceinline__ int damped_solve(const MA &Ms, T par, const T (&g)[P], float thr,
+template <int P, typename T, bool ESC, bool LSM, typename MA>
+__device__ __forceinline__ int damped_solve(const MA &Ms, T par, const T (&v)[P], const T (&invD)[P], bool fuse, float thr,
                                             T (&z)[P], T &znorm, T &w2, T &minpiv, unsigned &n_esc,
                                             T *lslot)
 {
     // FP64 solves take no pivot threshold (there is no higher precision to
     // escalate to), so only FP32 solves can return 1
-    int rc = chol_solve<P, T, T>(Ms, par, g, (ESC && sizeof(T) == 4) ? (T)thr : T(0), z, znorm, w2, minpiv,
-                                 lslot);
+    int rc = chol_solve<P, T, T, LSM>(Ms, par, v, invD, fuse, (ESC && sizeof(T) == 4) ? (T)thr : T(0), z, znorm, w2,
+                                      minpiv, lslot);
     if constexpr (ESC && sizeof(T) == 4) {
         if (rc == 1) {
             ++n_esc;
-            float msl[tri(P)], gl[P], zl[P], o2[2];
+            float msl[tri(P)], vl[P], dl[P], zl[P], o2[2];
 #pragma unroll
             for (int k = 0; k < tri(P); ++k) msl[k] = Ms[k];
 #pragma unroll
-            for (int k = 0; k < P; ++k) gl[k] = g[k];
-            rc = chol_solve_fp64<P>(msl, par, gl, zl, o2);
+            for (int k = 0; k < P; ++k) {
+                vl[k] = v[k];
+                dl[k] = invD[k];
+            }
+            rc = chol_solve_fp64<P>(msl, par, vl, dl, zl, o2);
 #pragma unroll
             for (int k = 0; k < P; ++k) z[k] = zl[k];
             znorm = o2[0];
@@ -606,8 +667,8 @@ __device__ __forceinline__ int damped_solve(const MA &Ms, T par, const T (&g)[P]
 // quantity and the threshold of a branch it decided (the Newton acceptance
 // fp <= 0.1 delta, the |fp| <= 0.1 delta stop, the fp <= fp_old stop): a
 // small margin means a rounding difference could have taken the other branch.
-template <int P, typename T, bool ESC, typename MA>
-__device__ __forceinline__ void lmpar_scaled(const MA &Ms, const T (&g)[P], T delta, T &par,
+template <int P, typename T, bool ESC, bool LSM, typename MA>
+__device__ __forceinline__ void lmpar_scaled(const MA &Ms, const T (&v)[P], const T (&invD)[P], int fuse, T delta, T &par,
                                              T (&z)[P], float thr, unsigned &n_lambda, unsigned &n_esc,
                                              bool &singular, T &newton_piv, T &margin, T *lslot = nullptr)
 {
@@ -627,7 +688,7 @@ __device__ __forceinline__ void lmpar_scaled(const MA &Ms, const T (&g)[P], T de
             pr = t > tiny_pos<T>() ? t : tiny_pos<T>();
         }
         ++n_lambda;
-        const int rc = damped_solve<P, T, ESC>(Ms, pr, g, thr, z, dxnorm, w2, mp, n_esc, lslot);
+        const int rc = damped_solve<P, T, ESC, LSM>(Ms, pr, v, invD, ((first ? fuse : fuse >> 1) & 1) != 0, thr, z, dxnorm, w2, mp, n_esc, lslot);
         if (first) {
             first = false;
             newton_piv = mp;
@@ -645,9 +706,11 @@ __device__ __forceinline__ void lmpar_scaled(const MA &Ms, const T (&g)[P], T de
                 return;
             }
             par_l = (!rank_def && w2 > T(0)) ? fdiv(fp * idelta, w2) : T(0);
-            T gn2 = T(0);
+            T gn2 = T(0), g0 = T(0);
 #pragma unroll
-            for (int i = 0; i < P; ++i) gn2 += g[i] * g[i];
+            for (int i = 0; i < P; ++i) {
+                add_square<T>(mul_rn(v[i], invD[i]), i, g0, gn2);
+            }
             gnorm = fsqrt(gn2);
             par_u = gnorm * idelta;
             if (par_u == T(0)) par_u = tiny_pos<T>() / (delta < T(0.1) ? delta : T(0.1));

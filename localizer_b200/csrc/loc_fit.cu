@@ -24,13 +24,15 @@ namespace {
 
 constexpr unsigned kFull = 0xffffffffu;
 constexpr int K = kMaxHalfWidth + 1;
-constexpr int M_NCLS = 0, M_MAXR = 1;
+// header: ROI classes present, largest half-width; length and dequeue cursor
+// of the queue, of the fits past the first level's budget, and of the fits
+// left to the teams. The FP64 re-run's tables (meta2, meta3) use the first
+// and the last pair.
+constexpr int M_NCLS = 0, M_MAXR = 1, M_TOTAL = 2, M_NEXT = 3, M_NCONT = 4, M_CONTNEXT = 5, M_NLEFT = 6, M_LEFTNEXT = 7;
 // per ROI half-width r: queue start, count, dequeue cursor, histogram, fill cursor
 __host__ __device__ constexpr int m_start(int r) { return 8 + 1 * K + r; }
 __host__ __device__ constexpr int m_count(int r) { return 8 + 2 * K + r; }
 __host__ __device__ constexpr int m_next(int r) { return 8 + 3 * K + r; }
-__host__ __device__ constexpr int m_ccount(int r) { return 8 + 6 * K + r; }
-__host__ __device__ constexpr int m_cnext(int r) { return 8 + 7 * K + r; }
 __host__ __device__ constexpr int m_hist(int r) { return 8 + 4 * K + r; }
 __host__ __device__ constexpr int m_fill(int r) { return 8 + 5 * K + r; }
 
@@ -120,6 +122,7 @@ __global__ void k0_classes(int *meta)
     }
     meta[M_NCLS] = ncls;
     meta[M_MAXR] = maxr;
+    meta[M_TOTAL] = start;
 }
 
 __global__ void k0_scatter(const int *cls, int n, int *meta, int *order)
@@ -138,111 +141,89 @@ __global__ void k0_scatter(const int *cls, int n, int *meta, int *order)
     order[base + __popc(peers & ((1u << lane) - 1))] = i;
 }
 
+// Appends i of the lanes with want to a list, one atomic per warp.
+__device__ __forceinline__ void push(bool want, int i, int *list, int *count)
+{
+    const unsigned who = __ballot_sync(kFull, want);
+    if (!who) return;
+    const int lane = threadIdx.x & 31, first = __ffs(who) - 1;
+    int at = 0;
+    if (lane == first) at = atomicAdd(count, __popc(who));
+    at = __shfl_sync(kFull, at, first);
+    if (want) list[at + __popc(who & ((1u << lane) - 1))] = i;
+}
+
 // Fits of the FP32 solver whose result could depend on its rounding go to an
 // FP64 re-run: a branch decision of the trust-region method was within
 // `margin` of its threshold, the undamped normal matrix had a pivot ratio
-// below `pivot` (ill-conditioned), or the solver stopped for lack of
-// progress.
+// below `pivot` (ill-conditioned), the solver stopped for lack of progress, or
+// one of the options' rules holds. Walks the queue and appends them to order2
+// / meta2, or, when their FP32 solve took more than long_iters iterations and
+// a long queue exists, to order3 / meta3: the long fits set the length of the
+// re-run, so they are dequeued first.
 template <int P>
-__global__ void k3_flag(const float *state32, int stride, const int *cls, const uint8_t *flags, int n, float margin,
-                        float pivot, int *cls2, int *meta2)
-{
-    using SL = StateLayout<P>;
-    __shared__ int hist[K];
-    for (int r = threadIdx.x; r < K; r += blockDim.x) hist[r] = 0;
-    __syncthreads();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) {
-        int c2 = -1;
-        if (cls[i] >= 0 && flags[i] == F_PENDING) {
-            const float *s = state32 + (size_t)i * stride;
-            // fits stopped by the iteration cap are left alone: they have not
-            // converged, are almost always rejected, and cost 200 iterations
-            const float status = s[SL::STATUS];
-            const bool risky = status != (float)T_MAX_ITER &&
-                               (s[SL::MARGIN] < margin || s[SL::MINPIV] < pivot || status != 0.0f);
-            if (risky) {
-                c2 = cls[i];
-                atomicAdd(&hist[c2], 1);
-            }
-        }
-        cls2[i] = c2;
-    }
-    __syncthreads();
-    for (int r = threadIdx.x; r < K; r += blockDim.x)
-        if (hist[r]) atomicAdd(&meta2[m_hist(r)], hist[r]);
-}
-
-// Per-class form of the flag pass: walks the queue of half-width r and
-// appends the flagged fits to that class's FP64 queue (order2 / meta2), or,
-// when their FP32 solve took more than long_iters iterations and a long
-// queue exists (order3 / meta3), to that one: the long fits set the length
-// of the re-run, so they get their own launch with more threads per fit.
-template <int P>
-__global__ void k3_flag_class(const float *state32, int stride, const int *order, const int *meta,
-                              const uint8_t *flags, int r, float margin, float pivot, int warm_limit, int *cls2,
-                              int *order2, int *meta2, int long_iters, int *order3, int *meta3, int capped,
-                              float cond, int iters_min, float skip_rej, float w0)
+__global__ void k3_flag(const float *state32, int stride, const int *order, const int *meta, const int *cls,
+                        const uint8_t *flags, float margin, float pivot, int warm_limit, int *cls2,
+                        int *order2, int *meta2, int long_iters, int *order3, int *meta3, int capped,
+                        float cond, int iters_min, float skip_rej, float w0)
 {
     using SL = StateLayout<P>;
     constexpr int IX = P == 5 ? 2 : P == 4 ? 1 : 3;
-    const int start = meta[m_start(r)], count = meta[m_count(r)];
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        meta2[m_start(r)] = start;
-        if (meta3) meta3[m_start(r)] = start;
-    }
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < count; t += gridDim.x * blockDim.x) {
-        const int i = order[start + t];
-        if (flags[i] != F_PENDING) continue;
-        const float *s = state32 + (size_t)i * stride;
-        const float status = s[SL::STATUS];
-        // warm-started fits (warm_limit > 0) that needed many iterations may
-        // stop elsewhere than the reference start's trajectory would
-        // capped: fits the FP32 solver stopped at the iteration cap are
-        // re-run too (the FP64 solve may converge where FP32 did not)
-        const bool is_capped = status == (float)T_MAX_ITER;
-        // cond > 0: a branch margin is also too small when it is within the
-        // FP32 error the fit's conditioning allows (cond * eps32 / smallest
-        // undamped pivot ratio)
-        const float mthr = cond > 0.0f ? fmaxf(margin, cond * 5.96e-8f / fmaxf(s[SL::MINPIV], 1e-30f)) : margin;
-        const bool risky = is_capped ? capped != 0
-                                     : (s[SL::MARGIN] < mthr || s[SL::MINPIV] < pivot || status != 0.0f ||
-                                        (warm_limit > 0 && s[SL::ITERS] > (float)warm_limit) ||
-                                        (iters_min > 0 && s[SL::ITERS] >= (float)iters_min));
-        // skip_rej > 0: a fit whose FP32 end point lies clearly inside a reject
-        // rule of the finaliser (centre more than skip_rej px outside the ROI,
-        // amplitude below zero by more than skip_rej of its start scale, or
-        // every width more than the fraction skip_rej outside its accepted
-        // range) is not re-run: only its reject code could change
-        bool clear_reject = false;
-        if (risky && skip_rej > 0.0f) {
-            const float side = (float)(2 * r);
-            const float x = s[IX], y = s[IX + 1], A = s[0];
-            clear_reject = x < -skip_rej || x > side + skip_rej || y < -skip_rej || y > side + skip_rej ||
-                           A < -skip_rej * fmaxf(fabsf(s[P - 1]), 1.0f);
-            const float lo = 0.4f * w0 * (1.0f - skip_rej), hi = 1.5f * w0 * (1.0f + skip_rej);
-            if constexpr (P == 5) {
-                const float wd = fabsf(s[1]);
-                clear_reject = clear_reject || wd < lo || wd > hi;
-            } else if constexpr (P == 7) {
-                // axes of the covariance [[sx^2, rho sx sy], [rho sx sy, sy^2]]
-                const float sx = fabsf(s[1]), sy = fabsf(s[2]), rho = s[5];
-                const float a = sx * sx, c = sy * sy, b = rho * sx * sy;
-                const float ht = 0.5f * (a + c), rad = sqrtf(0.25f * (a - c) * (a - c) + b * b);
-                const float s1 = sqrtf(fmaxf(ht - rad, 0.0f)), s2 = sqrtf(ht + rad);
-                clear_reject = clear_reject || ((s1 < lo || s1 > hi) && (s2 < lo || s2 > hi));
+    const int count = meta[M_TOTAL];
+    // whole warps walk together (push)
+    for (int t0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); t0 < count; t0 += gridDim.x * blockDim.x) {
+        const int t = t0 + (int)(threadIdx.x & 31);
+        const int i = t < count ? order[t] : 0;
+        const int r = t < count ? cls[i] : 0;
+        bool rerun = false, is_long = false;
+        if (t < count && flags[i] == F_PENDING) {
+            const float *s = state32 + (size_t)i * stride;
+            const float status = s[SL::STATUS];
+            // warm-started fits (warm_limit > 0) that needed many iterations may
+            // stop elsewhere than the reference start's trajectory would
+            // capped: fits the FP32 solver stopped at the iteration cap are
+            // re-run too (the FP64 solve may converge where FP32 did not)
+            const bool is_capped = status == (float)T_MAX_ITER;
+            // cond > 0: a branch margin is also too small when it is within the
+            // FP32 error the fit's conditioning allows (cond * eps32 / smallest
+            // undamped pivot ratio)
+            const float mthr = cond > 0.0f ? fmaxf(margin, cond * 5.96e-8f / fmaxf(s[SL::MINPIV], 1e-30f)) : margin;
+            const bool risky = is_capped ? capped != 0
+                                         : (s[SL::MARGIN] < mthr || s[SL::MINPIV] < pivot || status != 0.0f ||
+                                            (warm_limit > 0 && s[SL::ITERS] > (float)warm_limit) ||
+                                            (iters_min > 0 && s[SL::ITERS] >= (float)iters_min));
+            // skip_rej > 0: a fit whose FP32 end point lies clearly inside a reject
+            // rule of the finaliser (centre more than skip_rej px outside the ROI,
+            // amplitude below zero by more than skip_rej of its start scale, or
+            // every width more than the fraction skip_rej outside its accepted
+            // range) is not re-run: only its reject code could change
+            bool clear_reject = false;
+            if (risky && skip_rej > 0.0f) {
+                const float side = (float)(2 * r);
+                const float x = s[IX], y = s[IX + 1], A = s[0];
+                clear_reject = x < -skip_rej || x > side + skip_rej || y < -skip_rej || y > side + skip_rej ||
+                               A < -skip_rej * fmaxf(fabsf(s[P - 1]), 1.0f);
+                const float lo = 0.4f * w0 * (1.0f - skip_rej), hi = 1.5f * w0 * (1.0f + skip_rej);
+                if constexpr (P == 5) {
+                    const float wd = fabsf(s[1]);
+                    clear_reject = clear_reject || wd < lo || wd > hi;
+                } else if constexpr (P == 7) {
+                    // axes of the covariance [[sx^2, rho sx sy], [rho sx sy, sy^2]]
+                    const float sx = fabsf(s[1]), sy = fabsf(s[2]), rho = s[5];
+                    const float a = sx * sx, c = sy * sy, b = rho * sx * sy;
+                    const float ht = 0.5f * (a + c), rad = sqrtf(0.25f * (a - c) * (a - c) + b * b);
+                    const float s1 = sqrtf(fmaxf(ht - rad, 0.0f)), s2 = sqrtf(ht + rad);
+                    clear_reject = clear_reject || ((s1 < lo || s1 > hi) && (s2 < lo || s2 > hi));
+                }
+            }
+            if (risky && !clear_reject) {
+                cls2[i] = r;
+                rerun = true;
+                is_long = meta3 && s[SL::ITERS] > (float)long_iters;
             }
         }
-        if (risky && !clear_reject) {
-            cls2[i] = r;
-            if (meta3 && s[SL::ITERS] > (float)long_iters) {
-                const int slot = atomicAdd(&meta3[m_count(r)], 1);
-                order3[start + slot] = i;
-            } else {
-                const int slot = atomicAdd(&meta2[m_count(r)], 1);
-                order2[start + slot] = i;
-            }
-        }
+        push(rerun && !is_long, i, order2, &meta2[M_TOTAL]);
+        if (meta3) push(is_long, i, order3, &meta3[M_TOTAL]);
     }
 }
 
@@ -263,10 +244,20 @@ struct K1Args {
     float pivot_thr;
     const float *init_params;
     unsigned long long *stats;
-    int level;          // 0: fresh candidates, 1: fits suspended by level 0
-    int budget;         // level-0 iteration budget (0: none)
-    int *cont;          // continuation queue, laid out like order
-    float *cont_state;  // saved solver state of suspended fits
+    // list mode (r = 0): a list of candidates of any ROI size instead of one
+    // class's part of the queue
+    const int *list, *count;
+    int *next;
+    const int *cls;
+    int resume;         // the list's fits are suspended ones
+    int least;          // lists of at most this many fits are left to the teams
+    int budget;         // iterations a fit may use (0: all)
+    int drain;          // a warp whose queue is empty hands its fits over when at most this many
+                        // of its groups still have one
+    int *cont, *n_cont;     // fits past the budget
+    int *left, *n_left;     // fits left to the teams (entry k at left[k * left_step])
+    int left_step;
+    float *cont_state;  // saved solver state of both (see save_state)
     int cont_stride;
     int compensated;    // FP32 solver: sum the group's partial normal equations in FP64
     const int *roi_slot;  // ROI mode: first pixel of each candidate's packed ROI (row pitch 2r + 1)
@@ -329,61 +320,144 @@ __device__ __forceinline__ T group_max(T v, int tpf, unsigned mask)
     return v;
 }
 
-// Saved solver state of a suspended fit (continuation level), floats:
-// parameters, J^T J, J^T f, D, last step, then 11 scalars.
+// Saved solver state of a suspended fit: parameters, J^T J, J^T f, D, last
+// step, then scalars. FP32 fits keep it in cont_state (floats). An FP64 fit
+// keeps parameters and J^T J where its result goes, the scalars behind them,
+// and the three vectors in its cont_state record (free once its FP32 solve is
+// done), as doubles.
 template <int P> struct ContLayout {
     static constexpr int NT = tri(P);
     static constexpr int TH = 0, A = P, V = P + NT, D = 2 * P + NT, DX = 3 * P + NT, SC = 4 * P + NT;
     static constexpr int STRIDE = ((SC + 11) + 3) / 4 * 4;
+    static_assert(P + NT + 9 <= StateLayout<P>::STRIDE && 3 * P * 2 <= STRIDE, "FP64 state of a suspended fit");
+};
+template <typename T> struct Scalars {
+    T fnorm, delta, par, xnorm, minpiv, margin;
+    int it_state, iterations, xo, yo, q_n;   // q_n: partial sums the fit runs with (FP64)
+    unsigned esc;
 };
 
+// where a suspended fit's arrays are
+template <typename T> struct Saved {
+    T *th, *v, *D, *dx, *A, *sc;
+};
+template <int P, typename T>
+__device__ __forceinline__ Saved<T> saved_of(float *cont_state, int cont_stride, void *state, int state_stride, int i)
+{
+    using CL = ContLayout<P>;
+    if constexpr (sizeof(T) == 4) {
+        float *o = cont_state + (size_t)i * cont_stride;
+        return Saved<T>{o + CL::TH, o + CL::V, o + CL::D, o + CL::DX, o + CL::A, o + CL::SC};
+    } else {
+        double *s = (double *)state + (size_t)i * state_stride;
+        double *o = reinterpret_cast<double *>(cont_state + (size_t)i * cont_stride);
+        return Saved<T>{s, o, o + P, o + 2 * P, s + P, s + P + CL::NT};
+    }
+}
+template <typename T> __device__ __forceinline__ void save_scalars(T *o, const Scalars<T> &c)
+{
+    o[0] = c.fnorm;
+    o[1] = c.delta;
+    o[2] = c.par;
+    o[3] = c.xnorm;
+    o[4] = c.minpiv;
+    o[5] = c.margin;
+    if constexpr (sizeof(T) == 4) {
+        o[6] = __int_as_float(c.it_state);
+        o[7] = __int_as_float(c.iterations);
+        o[8] = __int_as_float(c.xo);
+        o[9] = __int_as_float(c.yo);
+        o[10] = __uint_as_float(c.esc);
+    } else {   // small integers, exact
+        o[6] = (double)((long long)c.iterations * 32 + (c.it_state == 1 ? 16 : 0) + c.q_n);
+        o[7] = (double)c.xo;
+        o[8] = (double)c.yo;
+    }
+}
+template <typename T> __device__ __forceinline__ Scalars<T> load_scalars(const T *o)
+{
+    Scalars<T> c;
+    c.fnorm = o[0];
+    c.delta = o[1];
+    c.par = o[2];
+    c.xnorm = o[3];
+    c.minpiv = o[4];
+    c.margin = o[5];
+    if constexpr (sizeof(T) == 4) {
+        c.it_state = __float_as_int(o[6]);
+        c.iterations = __float_as_int(o[7]);
+        c.xo = __float_as_int(o[8]);
+        c.yo = __float_as_int(o[9]);
+        c.esc = __float_as_uint(o[10]);
+        c.q_n = 0;
+    } else {
+        const long long w = (long long)o[6];
+        c.it_state = w & 16 ? 1 : 2;   // the solver asks only whether it is the first
+        c.q_n = (int)(w & 15);
+        c.iterations = (int)(w >> 5);
+        c.xo = (int)o[7];
+        c.yo = (int)o[8];
+        c.esc = 0;
+    }
+    return c;
+}
 
-// Shared memory of the solver block: the ROIs, then (FP64 only) the
-// per-fit normal equations.
+}  // namespace
+}  // namespace locb
+#include "loc_team.cuh"
+namespace locb {
+namespace {
+
+// Shared memory of one fit of the solver block: its ROI, then (FP64 only) its
+// state and matrices.
 template <typename T>
 __host__ __device__ constexpr int state_smem_per_fit(int P) { return sizeof(T) == 8 ? (3 * tri(P) + 5 * P) * 8 : 0; }
+template <typename T>
+__host__ __device__ constexpr int slot_bytes(int P, int r, int tpf)
+{
+    const int roi = roi_stride((2 * r + 1) * (2 * r + 1), tpf) * 4;
+    return sizeof(T) == 8 ? (roi + 15) / 16 * 16 + (state_smem_per_fit<T>(P) + 15) / 16 * 16 : roi;
+}
 
-// Process one queue of ROI half-width r: the fresh candidates (level 0) or
-// the fits suspended there (level 1). TPF threads cooperate on each fit;
+// Process one queue: the candidates of ROI half-width r, or (r = 0) a list of
+// fits of any size, fresh or suspended. TPF threads cooperate on each fit;
 // S = 2r + 1 at compile time, or 0 for a runtime side.
 template <int METHOD, typename T, int S, int TPF, bool ESC>
-__device__ __forceinline__ void run_class(const K1Args &a, int r, float *smem, unsigned (&st)[ST_N])
+__device__ __forceinline__ void run_class(const K1Args &a, int r_class, int smem_bytes, float *smem, unsigned (&st)[ST_N])
 {
     constexpr int P = Traits<METHOD>::P;
     constexpr int NT = tri(P);
     constexpr int IX = Traits<METHOD>::IX;
     using SL = StateLayout<P>;
-    using CL = ContLayout<P>;
     const int tid = threadIdx.x;
     const int lane = tid & 31;
     const int q = lane % TPF;            // sub-lane within the fit's group
     const int glead = lane - q;          // lane of the group leader
     const bool leader = q == 0;
-    const int s = S > 0 ? S : 2 * r + 1;
-    const int npx = s * s;
-    const int stride = roi_stride(npx, TPF);
-    const float *myroi = smem + (tid / TPF) * stride;
-    const bool cont = a.level == 1;
-    const int *queue = cont ? a.cont : a.order;
-    const int cstart = a.meta[m_start(r)];
-    const int ccount = a.meta[cont ? m_ccount(r) : m_count(r)];
-    int *next = a.meta + (cont ? m_cnext(r) : m_next(r));
+    const bool by_list = S == 0 && r_class == 0;
+    // in list mode every fit brings its own ROI size, and the block has as
+    // many groups as the largest one present lets into its shared memory
+    int r = by_list ? a.meta[M_MAXR] : r_class;
+    const int slot = slot_bytes<T>(P, r, TPF);
+    const bool has_room = !by_list || (tid / TPF + 1) * slot <= smem_bytes;
+    int s = S > 0 ? S : 2 * r + 1;
+    int npx = s * s;
+    const int stride = slot / 4;
+    float *myroi = smem + (tid / TPF) * stride;
+    const int *queue = by_list ? a.list : a.order + a.meta[m_start(r)];
+    const int ccount = by_list ? *a.count : a.meta[m_count(r)];
+    int *next = by_list ? a.next : a.meta + m_next(r);
     const T inv_s2 = sizeof(T) == 4 ? (T)a.inv_s2 : (T)a.inv_s2_d;
     const T inv_abs_s = sizeof(T) == 4 ? (T)a.inv_abs_s : (T)a.inv_abs_s_d;
     const T w0 = (T)a.w0;
 
+    // FP64: the normal equations, parameters, scaling, last step, the scaled
+    // matrix of the damped solve and its factor live in the fit's
+    // shared-memory slot (in registers they push the FP64 solver into spills)
     constexpr bool kSmemState = sizeof(T) == 8;
     T *sstate = nullptr;
-    if constexpr (kSmemState) {
-        const int roi_bytes = (blockDim.x / TPF) * stride * (int)sizeof(float);
-        // one slot of state_smem_per_fit bytes per fit (the group's threads share it)
-        sstate = (T *)((char *)smem + ((roi_bytes + 15) / 16) * 16) +
-                 (tid / TPF) * (state_smem_per_fit<T>(P) / (int)sizeof(T));
-    }
-    // FP64: the normal equations, parameters, scaling, last step and the
-    // scaled matrix of the damped solve live in the fit's shared-memory slot
-    // (in registers they push the FP64 solver into spills); te, the
-    // evaluation point, stays in registers
+    if constexpr (kSmemState)
+        sstate = (T *)((char *)myroi + slot - (state_smem_per_fit<T>(P) + 15) / 16 * 16);
     StateArr<T, NT, kSmemState> A(sstate);
     StateArr<T, P, kSmemState> v(sstate ? sstate + NT : nullptr);
     StateArr<T, P, kSmemState> th(sstate ? sstate + NT + P : nullptr);
@@ -395,11 +469,13 @@ __device__ __forceinline__ void run_class(const K1Args &a, int r, float *smem, u
     T minpiv_fit = T(1);
     T margin_fit = T(1e30);
     unsigned esc_fit = 0;
-    bool exhausted = false;
+    bool exhausted = !has_room;
+    if (!kSmemState || has_room) {
 #pragma unroll
-    for (int k = 0; k < P; ++k) th[k] = v[k] = D[k] = dx[k] = te[k] = T(0);
+        for (int k = 0; k < P; ++k) th[k] = v[k] = D[k] = dx[k] = te[k] = T(0);
 #pragma unroll
-    for (int k = 0; k < NT; ++k) A[k] = T(0);
+        for (int k = 0; k < NT; ++k) A[k] = T(0);
+    }
 
     auto theta_abs = [&](int k, auto &t) -> T {
         return k == IX ? t[k] + (T)xo : (k == IX + 1 ? t[k] + (T)yo : t[k]);
@@ -431,49 +507,35 @@ __device__ __forceinline__ void run_class(const K1Args &a, int r, float *smem, u
             st[ST_ITERS] += iterations;
         }
     };
-    // park a fit that used up the first level's iteration budget
-    auto write_suspend = [&]() {
+    // park a fit that used up its iteration budget, or whose warp has run dry
+    auto write_suspend = [&](bool over) {
         if (leader) {
-            float *o = a.cont_state + (size_t)cidx * a.cont_stride;
+            const Saved<T> o = saved_of<P, T>(a.cont_state, a.cont_stride, a.state, a.state_stride, cidx);
 #pragma unroll
             for (int k = 0; k < P; ++k) {
-                o[CL::TH + k] = (float)th[k];
-                o[CL::V + k] = (float)v[k];
-                o[CL::D + k] = (float)D[k];
-                o[CL::DX + k] = (float)dx[k];
+                o.th[k] = th[k];
+                o.v[k] = v[k];
+                o.D[k] = D[k];
+                o.dx[k] = dx[k];
             }
 #pragma unroll
-            for (int k = 0; k < NT; ++k) o[CL::A + k] = (float)A[k];
-            float *sc = o + CL::SC;
-            sc[0] = (float)fnorm;
-            sc[1] = (float)delta;
-            sc[2] = (float)par;
-            sc[3] = (float)xnorm;
-            sc[4] = __int_as_float(it_state);
-            sc[5] = __int_as_float(iterations);
-            sc[6] = (float)minpiv_fit;
-            sc[7] = (float)margin_fit;
-            sc[8] = __uint_as_float(esc_fit);
-            sc[9] = __int_as_float(xo);
-            sc[10] = __int_as_float(yo);
-            const int slot = atomicAdd(a.meta + m_ccount(r), 1);
-            a.cont[cstart + slot] = cidx;
+            for (int k = 0; k < NT; ++k) o.A[k] = A[k];
+            save_scalars<T>(o.sc, Scalars<T>{fnorm, delta, par, xnorm, minpiv_fit, margin_fit, it_state, iterations, xo,
+                                             yo, TPF, esc_fit});
+            if (over) a.cont[atomicAdd(a.n_cont, 1)] = cidx;
+            else a.left[atomicAdd(a.n_left, 1) * a.left_step] = cidx;
         }
     };
     // finish() and suspend() only mark the fit; its state is written at the
     // next flush(), before the lane is refilled (one inlined copy of each
     // write-out instead of one per call site)
-    int done = -1;   // -1 nothing pending, -2 suspended, else the termination status
+    int done = -1;   // -1 nothing pending, -2 over the budget, -3 left to the teams, else the termination status
     auto finish = [&](int status) {
         done = status;
         phase = 0;
     };
-    auto suspend = [&]() {
-        done = -2;
-        phase = 0;
-    };
     auto flush = [&]() {
-        if (done == -2) write_suspend();
+        if (done == -2 || done == -3) write_suspend(done == -2);
         else if (done >= 0) write_finish(done);
         done = -1;
     };
@@ -490,9 +552,14 @@ __device__ __forceinline__ void run_class(const K1Args &a, int r, float *smem, u
         margin_fit = fmin(margin_fit, fabs(worst - T(1)));
         return ok;
     };
+    bool drain = false;
     auto start_iteration = [&]() {
-        if (!cont && a.budget > 0 && iterations >= a.budget) {
-            suspend();
+        if (a.budget > 0 && iterations >= a.budget) {
+            finish(-2);
+            return;
+        }
+        if (drain) {
+            finish(-3);
             return;
         }
         ++iterations;
@@ -528,7 +595,7 @@ __device__ __forceinline__ void run_class(const K1Args &a, int r, float *smem, u
             int my = -1;
             if (want) {
                 const int qi = base + __popc(need & ((1u << glead) - 1));
-                if (qi < ccount) my = queue[cstart + qi];
+                if (qi < ccount) my = queue[qi];
                 else exhausted = true;
             }
             int fr = 0;
@@ -538,30 +605,35 @@ __device__ __forceinline__ void run_class(const K1Args &a, int r, float *smem, u
                 const double cx = cd.x, cy = cd.y, cint = cd.intensity, cbg = cd.background;
                 fr = cd.frame;
                 cidx = my;
-                if (cont) {
-                    const float *o = a.cont_state + (size_t)my * a.cont_stride;
+                if (by_list) {
+                    r = a.cls[my];
+                    s = 2 * r + 1;
+                    npx = s * s;
+                }
+                if (by_list && a.resume) {
+                    const Saved<T> o = saved_of<P, T>(a.cont_state, a.cont_stride, a.state, a.state_stride, my);
 #pragma unroll
                     for (int k = 0; k < P; ++k) {
-                        th[k] = (T)o[CL::TH + k];
-                        v[k] = (T)o[CL::V + k];
-                        D[k] = (T)o[CL::D + k];
-                        dx[k] = (T)o[CL::DX + k];
+                        th[k] = o.th[k];
+                        v[k] = o.v[k];
+                        D[k] = o.D[k];
+                        dx[k] = o.dx[k];
                     }
 #pragma unroll
-                    for (int k = 0; k < NT; ++k) A[k] = (T)o[CL::A + k];
-                    const float *sc = o + CL::SC;
-                    fnorm = (T)sc[0];
-                    delta = (T)sc[1];
-                    par = (T)sc[2];
-                    xnorm = (T)sc[3];
-                    it_state = __float_as_int(sc[4]);
-                    iterations = __float_as_int(sc[5]);
-                    minpiv_fit = (T)sc[6];
-                    margin_fit = (T)sc[7];
-                    esc_fit = __float_as_uint(sc[8]);
-                    xo = __float_as_int(sc[9]);
-                    yo = __float_as_int(sc[10]);
-                    phase = 3;  // resume: start the next outer iteration after staging
+                    for (int k = 0; k < NT; ++k) A[k] = o.A[k];
+                    const Scalars<T> c = load_scalars<T>(o.sc);
+                    fnorm = c.fnorm;
+                    delta = c.delta;
+                    par = c.par;
+                    xnorm = c.xnorm;
+                    minpiv_fit = c.minpiv;
+                    margin_fit = c.margin;
+                    it_state = c.it_state;
+                    iterations = c.iterations;
+                    xo = c.xo;
+                    yo = c.yo;
+                    esc_fit = c.esc;
+                    phase = 3;   // start the next outer iteration after staging
                 } else {
                     xo = (int)floor(cx - (double)r);
                     yo = (int)floor(cy - (double)r);
@@ -570,7 +642,7 @@ __device__ __forceinline__ void run_class(const K1Args &a, int r, float *smem, u
                     esc_fit = 0;
                     if (a.init_params && !isnan(a.init_params[(size_t)my * P])) {
                         const float *ip = a.init_params + (size_t)my * P;
-#pragma unroll
+    #pragma unroll
                         for (int k = 0; k < P; ++k) {
                             const double off = k == IX ? (double)xo : (k == IX + 1 ? (double)yo : 0.0);
                             th[k] = (T)((double)ip[k] - off);
@@ -593,22 +665,26 @@ __device__ __forceinline__ void run_class(const K1Args &a, int r, float *smem, u
             }
             // warp-cooperative ROI staging: global uint16 -> shared float
             unsigned got = __ballot_sync(kFull, my >= 0 && leader);
-            const int pitch = a.roi_slot ? s : a.n_rows;   // a packed ROI's rows are 2r + 1 pixels apart
             while (got) {
                 const int src = __ffs(got) - 1;
                 got &= got - 1;
                 const long long sbase = __shfl_sync(kFull, rbase, src);
+                const int side = S > 0 ? S : __shfl_sync(kFull, s, src);
+                const int pitch = a.roi_slot ? side : a.n_rows;   // a packed ROI's rows are 2r + 1 pixels apart
                 const uint16_t *fb = a.frames + sbase;
                 float *dst = smem + ((tid - lane + src) / TPF) * stride;
-                for (int k = lane; k < npx; k += 32) {
-                    const int j = k / s, i = k - j * s;
+                for (int k = lane; k < side * side; k += 32) {
+                    const int j = k / side, i = k - j * side;
                     dst[k] = (float)__ldg(fb + i + (size_t)j * pitch);
                 }
             }
             __syncwarp();
         }
-        // fits resumed from level 0 and fits whose last step was accepted
-        // start their next outer iteration here (one inlined copy of it)
+        // few fits left and none to refill with: hand them over
+        drain = a.drain > 0 && __ballot_sync(kFull, exhausted && has_room) != 0 &&
+                __popc(__ballot_sync(kFull, phase != 0 && leader)) <= a.drain;
+        // fits whose last step was accepted start their next outer iteration
+        // here (one inlined copy of it)
         if (phase == 3) start_iteration();
         if (__ballot_sync(kFull, phase != 0) == 0) break;
         lap(c_refill);
@@ -621,13 +697,10 @@ __device__ __forceinline__ void run_class(const K1Args &a, int r, float *smem, u
             do_pass = true;
         } else if (phase == 2) {
             ++trial;
-            T invD[P], g[P], z[P];
+            T invD[P], z[P];
             StateArr<T, NT, kSmemState> Ms(sstate ? sstate + NT + 4 * P : nullptr);
 #pragma unroll
-            for (int k = 0; k < P; ++k) {
-                invD[k] = frcp(D[k]);
-                g[k] = v[k] * invD[k];
-            }
+            for (int k = 0; k < P; ++k) invD[k] = frcp(D[k]);
 #pragma unroll
             for (int i = 0; i < P; ++i)
 #pragma unroll
@@ -635,8 +708,11 @@ __device__ __forceinline__ void run_class(const K1Args &a, int r, float *smem, u
             unsigned nl = 0, ne = 0;
             bool sing = false;
             T npiv;
-            lmpar_scaled<P, T, ESC>(Ms, g, delta, par, z, a.pivot_thr, nl, ne, sing, npiv, margin_fit,
-                                    sstate ? sstate + 2 * NT + 4 * P : nullptr);
+            T vr[P];
+#pragma unroll
+            for (int k = 0; k < P; ++k) vr[k] = v[k];
+            lmpar_scaled<P, T, ESC, kSmemState>(Ms, vr, invD, TPF == 1 || by_list ? sym_fuse(s, TPF) : 0, delta, par, z, a.pivot_thr, nl,
+                                    ne, sing, npiv, margin_fit, sstate ? sstate + 2 * NT + 4 * P : nullptr);
             if (leader) {
                 st[ST_LAMBDA] += nl;
                 st[ST_ESC] += ne;
@@ -761,10 +837,9 @@ __device__ __forceinline__ void run_class(const K1Args &a, int r, float *smem, u
                     }
                 }
                 const T if2 = frcp(fnorm * fnorm);
-                const T t1s = jdx2 * if2;
-                const T t2s = par * pnorm * pnorm * if2;
-                const T prered = t1s + T(2) * t2s;
-                const T dirder = -(t1s + t2s);
+                const T t2s = mul_rn(mul_rn(mul_rn(par, pnorm), pnorm), if2);
+                const T prered = fma(jdx2, if2, T(2) * t2s);
+                const T dirder = -fma(jdx2, if2, t2s);
                 const T ratio = prered > T(0) ? fdiv(actred, prered) : T(0);
                 margin_fit = fmin(margin_fit, fmin(fabs(ratio - T(0.25)), fmin(fabs(ratio - T(0.75)),
                                                                               fabs(ratio - T(1e-4)))));
@@ -844,13 +919,14 @@ __device__ __forceinline__ void run_class(const K1Args &a, int r, float *smem, u
 __host__ __device__ constexpr int k1_min_blocks(int method, int bytes) { return bytes == 8 ? 1 : (method == 7 ? 2 : 3); }
 
 template <int METHOD, typename T, int S, int TPF, bool ESC>
-__global__ void __launch_bounds__(128, k1_min_blocks(METHOD, sizeof(T))) k1_lm_fit(K1Args a, int r)
+__global__ void __launch_bounds__(128, k1_min_blocks(METHOD, sizeof(T))) k1_lm_fit(K1Args a, int r, int smem_bytes)
 {
     extern __shared__ float smem[];
     unsigned st[ST_N];
 #pragma unroll
     for (int k = 0; k < ST_N; ++k) st[k] = 0;
-    if (a.meta[a.level == 1 ? m_ccount(r) : m_count(r)] > 0) run_class<METHOD, T, S, TPF, ESC>(a, r, smem, st);
+    if (r > 0 ? a.meta[m_count(r)] > 0 : *a.count > a.least)
+        run_class<METHOD, T, S, TPF, ESC>(a, r, smem_bytes, smem, st);
     // warp-reduce the counters, one atomic per warp and counter
 #pragma unroll
     for (int k = 0; k < ST_N; ++k) {
@@ -1111,18 +1187,10 @@ __global__ void k2_finalize(K2Args a)
 
 int solver_method(int method) { return method == 5 ? 7 : method; }
 
-template <int METHOD, typename T, int S, int TPF, bool ESC = false>
-cudaError_t launch_k1_s(const K1Args &ka, int r, int tpb, int bps_req, cudaStream_t stream)
+// Blocks of a persistent kernel: every SM filled to its occupancy.
+template <typename F>
+cudaError_t persistent_grid(F *kern, int tpb, int smem, int bps_req, int *grid)
 {
-    auto kern = k1_lm_fit<METHOD, T, S, TPF, ESC>;
-    const int side = 2 * r + 1;
-    const int per_fit = roi_stride(side * side, TPF) * (int)sizeof(float);
-    constexpr int P = Traits<METHOD>::P;
-    auto smem_of = [&](int t) { return ((t / TPF) * per_fit + 15) / 16 * 16 + (t / TPF) * state_smem_per_fit<T>(P); };
-    // fewer threads per block when the block's shared memory would exceed 227 KB
-    while (tpb > 32 && smem_of(tpb) > 227 * 1024) tpb -= 32;
-    const int smem = smem_of(tpb);
-    if (smem > 227 * 1024) return cudaErrorInvalidValue;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
     int dev = 0, nsm = 0, bps = 0;
@@ -1132,51 +1200,137 @@ cudaError_t launch_k1_s(const K1Args &ka, int r, int tpb, int bps_req, cudaStrea
     if (e != cudaSuccess) return e;
     if (bps < 1) return cudaErrorInvalidConfiguration;
     if (bps_req > 0 && bps_req < bps) bps = bps_req;
-    kern<<<nsm * bps, tpb, smem, stream>>>(ka, r);
+    *grid = nsm * bps;
+    return cudaSuccess;
+}
+
+// r > 0: the class's queue; r = 0: a list, ROIs up to r_cap.
+template <int METHOD, typename T, int S, int TPF, bool ESC = false>
+cudaError_t launch_k1_s(const K1Args &ka, int r, int r_cap, int tpb, int bps_req, cudaStream_t stream)
+{
+    auto kern = k1_lm_fit<METHOD, T, S, TPF, ESC>;
+    const int slot = slot_bytes<T>(Traits<METHOD>::P, r > 0 ? r : r_cap, TPF);
+    int smem = (tpb / TPF) * slot;
+    if (r > 0) {
+        // fewer threads per block when the block's shared memory would exceed 227 KB
+        while (tpb > 32 && smem > 227 * 1024) {
+            tpb -= 32;
+            smem = (tpb / TPF) * slot;
+        }
+        if (smem > 227 * 1024) return cudaErrorInvalidValue;
+    } else {
+        // two blocks per SM; larger ROIs leave groups of a block without room
+        const int most = 113 * 1024;
+        if (slot > most) return cudaErrorInvalidValue;
+        if (smem > most) smem = most;
+    }
+    int grid = 0;
+    const cudaError_t e = persistent_grid(kern, tpb, smem, bps_req, &grid);
+    if (e != cudaSuccess) return e;
+    kern<<<grid, tpb, smem, stream>>>(ka, r, smem);
     return cudaGetLastError();
 }
 
-template <int METHOD, typename T, int TPF>
+template <int METHOD, int TPF>
 cudaError_t launch_k1_tpf(const K1Args &ka, int r, int tpb, int bps_req, cudaStream_t stream)
 {
-    if constexpr (sizeof(T) == 8) {
-        return launch_k1_s<METHOD, T, 0, TPF>(ka, r, tpb, bps_req, stream);
-    } else {
-        // FP64 pivot escalation: one runtime-side instantiation per method
-        // and threads per fit
-        if (ka.pivot_thr > 0.0f) return launch_k1_s<METHOD, T, 0, TPF, true>(ka, r, tpb, bps_req, stream);
-        switch (2 * r + 1) {
-        case 5: return launch_k1_s<METHOD, T, 5, TPF>(ka, r, tpb, bps_req, stream);
-        case 7: return launch_k1_s<METHOD, T, 7, TPF>(ka, r, tpb, bps_req, stream);
-        case 9: return launch_k1_s<METHOD, T, 9, TPF>(ka, r, tpb, bps_req, stream);
-        case 11: return launch_k1_s<METHOD, T, 11, TPF>(ka, r, tpb, bps_req, stream);
-        case 13: return launch_k1_s<METHOD, T, 13, TPF>(ka, r, tpb, bps_req, stream);
-        case 15: return launch_k1_s<METHOD, T, 15, TPF>(ka, r, tpb, bps_req, stream);
-        case 17: return launch_k1_s<METHOD, T, 17, TPF>(ka, r, tpb, bps_req, stream);
-        default: return launch_k1_s<METHOD, T, 0, TPF>(ka, r, tpb, bps_req, stream);
-        }
+    // FP64 pivot escalation: one runtime-side instantiation per method
+    // and threads per fit
+    if (ka.pivot_thr > 0.0f) return launch_k1_s<METHOD, float, 0, TPF, true>(ka, r, r, tpb, bps_req, stream);
+    switch (2 * r + 1) {
+    case 5: return launch_k1_s<METHOD, float, 5, TPF>(ka, r, r, tpb, bps_req, stream);
+    case 7: return launch_k1_s<METHOD, float, 7, TPF>(ka, r, r, tpb, bps_req, stream);
+    case 9: return launch_k1_s<METHOD, float, 9, TPF>(ka, r, r, tpb, bps_req, stream);
+    case 11: return launch_k1_s<METHOD, float, 11, TPF>(ka, r, r, tpb, bps_req, stream);
+    case 13: return launch_k1_s<METHOD, float, 13, TPF>(ka, r, r, tpb, bps_req, stream);
+    case 15: return launch_k1_s<METHOD, float, 15, TPF>(ka, r, r, tpb, bps_req, stream);
+    case 17: return launch_k1_s<METHOD, float, 17, TPF>(ka, r, r, tpb, bps_req, stream);
+    default: return launch_k1_s<METHOD, float, 0, TPF>(ka, r, r, tpb, bps_req, stream);
     }
 }
 
-// One persistent solver launch for the queue of half-width r with tpf
-// threads per fit (1, 4 or 8 for FP32; 1, 2, 4 or 8 for FP64).
-template <int METHOD, typename T>
-cudaError_t launch_k1(const K1Args &ka, int r, int tpb, int bps_req, int tpf, cudaStream_t stream)
+// One persistent first-level launch for the queue of half-width r with tpf
+// threads per fit (1, 4, 8 or 16).
+template <int METHOD>
+cudaError_t launch_first(const K1Args &ka, int r, int tpb, int bps_req, int tpf, cudaStream_t stream)
 {
-    if constexpr (sizeof(T) == 8) {
-        return tpf == 4 ? launch_k1_tpf<METHOD, T, 4>(ka, r, tpb, bps_req, stream)
-             : tpf == 8 ? launch_k1_tpf<METHOD, T, 8>(ka, r, tpb, bps_req, stream)
-             : tpf == 2 ? launch_k1_tpf<METHOD, T, 2>(ka, r, tpb, bps_req, stream)
-                        : launch_k1_tpf<METHOD, T, 1>(ka, r, tpb, bps_req, stream);
-    } else {
-        switch (tpf) {
-        case 4: return launch_k1_tpf<METHOD, T, 4>(ka, r, tpb, bps_req, stream);
-        case 8: return launch_k1_tpf<METHOD, T, 8>(ka, r, tpb, bps_req, stream);
-        // a half warp per fit (runtime ROI side only)
-        case 16: return launch_k1_s<METHOD, T, 0, 16>(ka, r, tpb, bps_req, stream);
-        default: return launch_k1_tpf<METHOD, T, 1>(ka, r, tpb, bps_req, stream);
-        }
+    switch (tpf) {
+    case 4: return launch_k1_tpf<METHOD, 4>(ka, r, tpb, bps_req, stream);
+    case 8: return launch_k1_tpf<METHOD, 8>(ka, r, tpb, bps_req, stream);
+    // a half warp per fit (runtime ROI side only)
+    case 16: return launch_k1_s<METHOD, float, 0, 16>(ka, r, r, tpb, bps_req, stream);
+    default: return launch_k1_tpf<METHOD, 1>(ka, r, tpb, bps_req, stream);
     }
+}
+
+// One launch over a list with tpf threads per fit (FP32: 1, 4 or 8; FP64: 1,
+// 2, 4 or 8).
+template <int METHOD, typename T>
+cudaError_t launch_list(const K1Args &ka, int r_cap, int tpb, int bps_req, int tpf, cudaStream_t stream)
+{
+    if constexpr (sizeof(T) == 4) {
+        if (ka.pivot_thr > 0.0f)
+            return tpf == 4 ? launch_k1_s<METHOD, T, 0, 4, true>(ka, 0, r_cap, tpb, bps_req, stream)
+                 : tpf == 8 ? launch_k1_s<METHOD, T, 0, 8, true>(ka, 0, r_cap, tpb, bps_req, stream)
+                            : launch_k1_s<METHOD, T, 0, 1, true>(ka, 0, r_cap, tpb, bps_req, stream);
+    } else {
+        if (tpf == 2) return launch_k1_s<METHOD, T, 0, 2>(ka, 0, r_cap, tpb, bps_req, stream);
+    }
+    return tpf == 4 ? launch_k1_s<METHOD, T, 0, 4>(ka, 0, r_cap, tpb, bps_req, stream)
+         : tpf == 8 ? launch_k1_s<METHOD, T, 0, 8>(ka, 0, r_cap, tpb, bps_req, stream)
+                    : launch_k1_s<METHOD, T, 0, 1>(ka, 0, r_cap, tpb, bps_req, stream);
+}
+template <typename T>
+cudaError_t launch_list_m(int m, const K1Args &ka, int r_cap, int tpb, int bps_req, int tpf, cudaStream_t stream)
+{
+    return m == 0 ? launch_list<0, T>(ka, r_cap, tpb, bps_req, tpf, stream)
+         : m == 1 ? launch_list<1, T>(ka, r_cap, tpb, bps_req, tpf, stream)
+                  : launch_list<7, T>(ka, r_cap, tpb, bps_req, tpf, stream);
+}
+
+// Calls of at most this many candidates run on the team solver alone: that is
+// two fits for every warp of a full device (148 SMs x 12 warps). With one
+// thread per fit such a call leaves most of the device idle for as long as its
+// longest fit takes (1 200 ellipsoidal fits 550 us, by teams 300 us).
+constexpr int kTeamOnlyFits = 3552;
+// Lists of at most this many fits go to the teams at once (FP32, FP64). FP32:
+// any value from 300 to 3552 measures the same; FP64: 3552 is the best of 1 to
+// 3552 at 20 000 to 520 000 fits a call.
+constexpr int kTeamFits32 = 3552, kTeamFits64 = 3552;
+// A warp that has run dry hands its last fits over at this many groups or
+// fewer: FP32 with one thread per fit (the ellipsoidal models, whose fits
+// differ most in length, keep them: measured 11.9 against 12.6 ms at 336 000
+// fits, while the symmetric ones lose 7.5 -> 7.8 ms without), the re-run with
+// two threads per fit, and FP64-precision calls.
+constexpr int kDrain1 = 4, kDrain2 = 3, kDrain64 = 8;
+
+template <int METHOD, typename T, bool ESC>
+cudaError_t launch_team_m(const TeamArgs &ta, int r_cap, int n_most, int bps_req, cudaStream_t stream)
+{
+    auto kern = k_team<METHOD, T, ESC>;
+    constexpr int tpb = 128, per_block = tpb / 32;
+    const int smem = per_block * team_smem<METHOD, T>(r_cap);
+    int grid = 0;
+    const cudaError_t e = persistent_grid(kern, tpb, smem, bps_req, &grid);
+    if (e != cudaSuccess) return e;
+    const int blocks = (n_most + per_block - 1) / per_block;
+    kern<<<blocks < grid ? blocks : grid, tpb, smem, stream>>>(ta, r_cap);
+    return cudaGetLastError();
+}
+
+// One team launch (method m of the solver) over at most n_most fits.
+template <typename T>
+cudaError_t launch_team(int m, const TeamArgs &ta, int r_cap, int n_most, int bps_req, cudaStream_t stream)
+{
+    if constexpr (sizeof(T) == 4) {
+        if (ta.k.pivot_thr > 0.0f)
+            return m == 0 ? launch_team_m<0, T, true>(ta, r_cap, n_most, bps_req, stream)
+                 : m == 1 ? launch_team_m<1, T, true>(ta, r_cap, n_most, bps_req, stream)
+                          : launch_team_m<7, T, true>(ta, r_cap, n_most, bps_req, stream);
+    }
+    return m == 0 ? launch_team_m<0, T, false>(ta, r_cap, n_most, bps_req, stream)
+         : m == 1 ? launch_team_m<1, T, false>(ta, r_cap, n_most, bps_req, stream)
+                  : launch_team_m<7, T, false>(ta, r_cap, n_most, bps_req, stream);
 }
 
 int cont_stride_of(int m) { return m == 0 ? ContLayout<5>::STRIDE : m == 1 ? ContLayout<4>::STRIDE : ContLayout<7>::STRIDE; }
@@ -1250,34 +1404,6 @@ void carve_scratch(void *base, int method, int n, int precision, int rerun, Scra
     s->init = warm ? (float *)p : nullptr;
 }
 
-namespace {
-
-template <typename T>
-cudaError_t launch_queues(const FitParams &p, const K1Args &k1_in, const int *counts, int r_cap, int tpb,
-                          bool two_level, int tpf_fixed, cudaStream_t stream, int *err_detail)
-{
-    K1Args k1 = k1_in;
-    const int m = solver_method(p.method);
-    cudaError_t e = cudaSuccess;
-    for (int level = 0; level < (two_level ? 2 : 1); ++level) {
-        k1.level = level;
-        k1.budget = two_level ? p.level0_budget : 0;
-        const int tpf = tpf_fixed > 0 ? tpf_fixed : (level == 0 ? p.threads_per_fit : p.tail_threads_per_fit);
-        for (int r = r_cap; r >= 1; --r) {
-            if (counts[r] <= 0) continue;
-            e = m == 0 ? launch_k1<0, T>(k1, r, tpb, p.blocks_per_sm, tpf, stream)
-              : m == 1 ? launch_k1<1, T>(k1, r, tpb, p.blocks_per_sm, tpf, stream)
-                       : launch_k1<7, T>(k1, r, tpb, p.blocks_per_sm, tpf, stream);
-            if (e == cudaErrorInvalidValue) *err_detail = 1;
-            if (e != cudaSuccess) return e;
-            if (p.launches) ++*p.launches;
-        }
-    }
-    return e;
-}
-
-}  // namespace
-
 cudaError_t enqueue_fit(const FitParams &p, const Scratch &s, cudaStream_t stream, int *err_detail)
 {
     *err_detail = 0;
@@ -1331,16 +1457,22 @@ cudaError_t enqueue_fit(const FitParams &p, const Scratch &s, cudaStream_t strea
     bump();
     bump();
 
-    // which half-width queues exist: known bound from the caller, or the
-    // histogram read back (one small synchronous copy)
+    // Calls of few fits run on the team solver alone: one launch over all ROI
+    // classes. Otherwise the first level runs a thread per fit, one launch
+    // per class that exists: known bound from the caller, or the histogram
+    // read back (one small synchronous copy).
+    const bool team_only = n <= kTeamOnlyFits && p.threads_per_fit == 1;
     int counts[K];
     for (int r = 0; r < K; ++r) counts[r] = r <= r_cap ? 1 : 0;
-    if (p.max_half_width <= 0) {
+    if (!team_only && p.max_half_width <= 0) {
         e = cudaMemcpyAsync(counts, s.meta + m_count(0), sizeof(int) * K, cudaMemcpyDeviceToHost, stream);
         if (e != cudaSuccess) return e;
         e = cudaStreamSynchronize(stream);
         if (e != cudaSuccess) return e;
     }
+    int r_most = 1;
+    for (int r = 1; r < K; ++r)
+        if (counts[r] > 0) r_most = r;
     mark(1);
     // learned start proposal and start check, before the solver chains fork
     if (p.warm) {
@@ -1354,110 +1486,171 @@ cudaError_t enqueue_fit(const FitParams &p, const Scratch &s, cudaStream_t strea
     if (tpb > 128) tpb = 128;
     const double s_abs = std::fabs(p.sigma);
     const int m = solver_method(p.method);
-    K1Args k1{px, px_frame, px_pitch, (const Cand *)p.cands, s.order, s.meta,
-              s.state, state_stride(p.method), (float)p.w0, (float)(1.0 / (p.sigma * p.sigma)),
-              (float)(1.0 / s_abs), 1.0 / (p.sigma * p.sigma), 1.0 / s_abs, p.max_iter, (float)p.epsabs,
-              (float)p.epsrel, p.precision == 1 ? 0.0f : p.pivot_thr, p.warm ? s.init : p.init_params, s.stats,
-              0, 0, s.cont, s.cont_state, cont_stride_of(m), p.compensated, p.roi_slot};
-    // Each ROI class is an independent chain -- level 0 (every candidate,
-    // tpf0 threads per fit, up to `budget` iterations), level 1 (the fits
-    // still running, tpf1 threads per fit), the flag pass and the FP64
-    // re-run of flagged fits -- forked onto the auxiliary streams so that the
-    // chains' tails overlap; the caller's stream joins them before the
-    // finaliser.
-    const bool two_level = p.precision != 1 && p.level0_budget > 0 && p.level0_budget < p.max_iter;
+    K1Args k1{};
+    k1.frames = px;
+    k1.frame_px = px_frame;
+    k1.n_rows = px_pitch;
+    k1.cands = (const Cand *)p.cands;
+    k1.order = s.order;
+    k1.meta = s.meta;
+    k1.state = s.state;
+    k1.state_stride = state_stride(p.method);
+    k1.w0 = (float)p.w0;
+    k1.inv_s2 = (float)(1.0 / (p.sigma * p.sigma));
+    k1.inv_abs_s = (float)(1.0 / s_abs);
+    k1.inv_s2_d = 1.0 / (p.sigma * p.sigma);
+    k1.inv_abs_s_d = 1.0 / s_abs;
+    k1.max_iter = p.max_iter;
+    k1.epsabs = (float)p.epsabs;
+    k1.epsrel = (float)p.epsrel;
+    k1.pivot_thr = p.precision == 1 ? 0.0f : p.pivot_thr;
+    k1.init_params = p.warm ? s.init : p.init_params;
+    k1.stats = s.stats;
+    k1.cls = s.cls;
+    k1.cont = s.cont;
+    k1.n_cont = s.meta + M_NCONT;
+    k1.left = s.cont + n - 1;   // from the other end of the list: a fit is in one of the two
+    k1.n_left = s.meta + M_NLEFT;
+    k1.left_step = -1;
+    k1.cont_state = s.cont_state;
+    k1.cont_stride = cont_stride_of(m);
+    k1.compensated = p.compensated;
+    k1.roi_slot = p.roi_slot;
+    // Auxiliary streams: independent launches run side by side so that their
+    // ends overlap; the caller's stream joins them.
     int naux = 0;
     while (naux < kMaxAux && p.aux[naux]) ++naux;
-    if (naux > 0) {
-        e = cudaEventRecord(p.fork, stream);
-        if (e != cudaSuccess) return e;
+    bool used[kMaxAux] = {false};
+    auto fork = [&]() -> cudaError_t { return naux > 0 ? cudaEventRecord(p.fork, stream) : cudaSuccess; };
+    auto side = [&](int j, cudaStream_t *cs) -> cudaError_t {
+        *cs = stream;
+        if (naux == 0) return cudaSuccess;
+        j %= naux;
+        *cs = p.aux[j];
+        const cudaError_t x = used[j] ? cudaSuccess : cudaStreamWaitEvent(*cs, p.fork, 0);
+        used[j] = true;
+        return x;
+    };
+    auto join = [&]() -> cudaError_t {
+        for (int j = 0; j < naux; ++j) {
+            if (!used[j]) continue;
+            used[j] = false;
+            cudaError_t x = cudaEventRecord(p.join[j], p.aux[j]);
+            if (x == cudaSuccess) x = cudaStreamWaitEvent(stream, p.join[j], 0);
+            if (x != cudaSuccess) return x;
+        }
+        return cudaSuccess;
+    };
+#define LOC_TRY(call) do { if ((e = (call)) != cudaSuccess) { if (e == cudaErrorInvalidValue) *err_detail = 1; return e; } bump(); } while (0)
+    cudaStream_t cs;
+    const bool fp64 = p.precision == 1;
+    const bool two_level = !fp64 && p.level0_budget > 0 && p.level0_budget < p.max_iter;
+    TeamArgs ta{};
+    ta.k = k1;
+    ta.switch_it = two_level ? p.level0_budget : p.max_iter;
+    ta.q0 = 1;
+    ta.q1 = p.tail_threads_per_fit;
+    ta.next = s.meta + M_LEFTNEXT;
+    const TeamList whole{s.order, s.meta + M_TOTAL, 1, 1, 0, n};
+    const TeamList left{s.cont + n - 1, s.meta + M_NLEFT, -1, 0, 0, n};
+    if (team_only) {
+        ta.list[0] = whole;
+        LOC_TRY(fp64 ? launch_team<double>(m, ta, r_most, n, p.blocks_per_sm, stream)
+                     : launch_team<float>(m, ta, r_most, n, p.blocks_per_sm, stream));
+    } else if (fp64) {
+        K1Args kf = k1;
+        kf.list = s.order;
+        kf.count = s.meta + M_TOTAL;
+        kf.next = s.meta + M_NEXT;
+        kf.drain = kDrain64;
+        LOC_TRY(launch_list_m<double>(m, kf, r_most, tpb, p.blocks_per_sm, 1, stream));
+        ta.list[0] = left;
+        LOC_TRY(launch_team<double>(m, ta, r_most, n, p.blocks_per_sm, stream));
+    } else {
+        // first level: the fresh candidates, one launch per ROI class
+        K1Args kf = k1;
+        kf.budget = two_level ? p.level0_budget : 0;
+        kf.drain = p.threads_per_fit == 1 && m != 7 ? kDrain1 : 0;
+        if ((e = fork()) != cudaSuccess) return e;
+        int chain = 0;
+        for (int r = r_most; r >= 1; --r) {
+            if (counts[r] <= 0) continue;
+            if ((e = side(chain++, &cs)) != cudaSuccess) return e;
+            LOC_TRY(m == 0 ? launch_first<0>(kf, r, tpb, p.blocks_per_sm, p.threads_per_fit, cs)
+                  : m == 1 ? launch_first<1>(kf, r, tpb, p.blocks_per_sm, p.threads_per_fit, cs)
+                           : launch_first<7>(kf, r, tpb, p.blocks_per_sm, p.threads_per_fit, cs));
+        }
+        if ((e = join()) != cudaSuccess || (e = fork()) != cudaSuccess) return e;
+        // second level: the fits past the budget; beside it the teams finish
+        // the fits that the first level's warps were left with (and the
+        // second level's, if they are few)
+        if (two_level) {
+            K1Args kl = k1;
+            kl.list = s.cont;
+            kl.count = s.meta + M_NCONT;
+            kl.next = s.meta + M_CONTNEXT;
+            kl.resume = 1;
+            kl.least = kTeamFits32;
+            if ((e = side(0, &cs)) != cudaSuccess) return e;
+            LOC_TRY(launch_list_m<float>(m, kl, r_most, tpb, p.blocks_per_sm, p.tail_threads_per_fit, cs));
+            ta.list[1] = TeamList{s.cont, s.meta + M_NCONT, 1, 0, 0, kTeamFits32};
+        }
+        ta.list[0] = left;
+        if ((e = side(1, &cs)) != cudaSuccess) return e;
+        LOC_TRY(launch_team<float>(m, ta, r_most, n, p.blocks_per_sm, cs));
+        if ((e = join()) != cudaSuccess) return e;
     }
-    bool used[kMaxAux] = {false}, used_long[kMaxAux] = {false};
-    int chain = 0;
-    for (int r = r_cap; r >= 1; --r) {
-        if (counts[r] <= 0) continue;
-        cudaStream_t cs = stream;
-        const int j = naux > 0 ? chain % naux : 0;
-        if (naux > 0) {
-            cs = p.aux[j];
-            if (!used[j]) {
-                if ((e = cudaStreamWaitEvent(cs, p.fork, 0)) != cudaSuccess) return e;
-                used[j] = true;
+    if (rerun) {
+        const int fb = n < 2 * 148 * 256 ? (n + 255) / 256 : 2 * 148;
+        const int wl = p.warm ? p.warm_iter_limit : 0;
+        const float *st32 = (const float *)s.state;
+        const int sst = state_stride(p.method);
+        int *o3 = long_q ? s.order3 : nullptr, *m3 = long_q ? s.meta3 : nullptr;
+        // a warm fit's reject says nothing about where the reference start's
+        // path ends: with a proposal every flagged fit is re-run
+        const float skip = p.warm ? 0.0f : p.rerun_skip_rejected;
+        auto flag = [&](auto kern) {
+            kern<<<fb, 256, 0, stream>>>(st32, sst, s.order, s.meta, s.cls, p.flags, p.rerun_margin, p.rerun_pivot, wl,
+                                         s.cls2, s.order2, s.meta2, p.long_rerun_iters, o3, m3, p.rerun_capped,
+                                         p.rerun_cond, p.rerun_iters, skip, (float)p.w0);
+            return cudaGetLastError();
+        };
+        LOC_TRY(m == 0 ? flag(k3_flag<5>) : m == 1 ? flag(k3_flag<4>) : flag(k3_flag<7>));
+        K1Args kd = k1;
+        kd.state = s.state64;
+        kd.stats = s.stats + ST_N;   // counters of the re-run kept apart
+        kd.pivot_thr = 0.0f;
+        if (p.warm) kd.init_params = nullptr;   // warm-started fits fall back to the reference start
+        kd.left = s.cont;                       // free again
+        kd.left_step = 1;
+        kd.n_left = s.meta2 + M_NLEFT;
+        kd.least = kTeamFits64;
+        ta.k = kd;
+        ta.switch_it = p.max_iter;
+        ta.next = s.meta2 + M_LEFTNEXT;
+        const int most = team_only ? n : kTeamFits64;
+        // the long re-runs first: they set the length of the launch
+        if (long_q) ta.list[0] = TeamList{s.order3, s.meta3 + M_TOTAL, 1, 1, p.long_rerun_threads_per_fit, most};
+        else ta.list[0] = TeamList{};
+        ta.list[1] = TeamList{s.order2, s.meta2 + M_TOTAL, 1, 1, p.rerun_threads_per_fit, most};
+        if (!team_only) {
+            // more flagged fits than the teams take: groups of threads first
+            if ((e = fork()) != cudaSuccess) return e;
+            for (int k = long_q ? 0 : 1; k < 2; ++k) {
+                const int tpf = k == 0 ? p.long_rerun_threads_per_fit : p.rerun_threads_per_fit;
+                kd.list = k == 0 ? s.order3 : s.order2;
+                kd.count = (k == 0 ? s.meta3 : s.meta2) + M_TOTAL;
+                kd.next = (k == 0 ? s.meta3 : s.meta2) + M_NEXT;
+                kd.drain = tpf <= 2 ? kDrain2 : 1;
+                if ((e = side(k, &cs)) != cudaSuccess) return e;
+                LOC_TRY(launch_list_m<double>(m, kd, r_most, tpb, p.blocks_per_sm, tpf, cs));
             }
+            if ((e = join()) != cudaSuccess) return e;
+            ta.list[2] = TeamList{s.cont, s.meta2 + M_NLEFT, 1, 0, 0, n};
         }
-        ++chain;
-        int cnt1[K];
-        for (int q = 0; q < K; ++q) cnt1[q] = q == r ? 1 : 0;
-        if (p.precision == 1) {
-            e = launch_queues<double>(p, k1, cnt1, r_cap, tpb, false, 1, cs, err_detail);
-        } else {
-            e = launch_queues<float>(p, k1, cnt1, r_cap, tpb, two_level, 0, cs, err_detail);
-            if (e == cudaSuccess && rerun) {
-                const int fb = 2 * 148;
-                const int wl = p.warm ? p.warm_iter_limit : 0;
-                const float *st32 = (const float *)s.state;
-                const int sst = state_stride(p.method);
-                int *o3 = long_q ? s.order3 : nullptr, *m3 = long_q ? s.meta3 : nullptr;
-                const int li = p.long_rerun_iters;
-                // a warm fit's reject says nothing about where the reference
-                // start's path ends: with a proposal every flagged fit is re-run
-                const float skip = p.warm ? 0.0f : p.rerun_skip_rejected;
-                switch (m) {
-                case 0: k3_flag_class<5><<<fb, 256, 0, cs>>>(st32, sst, s.order, s.meta, p.flags, r, p.rerun_margin,
-                                                             p.rerun_pivot, wl, s.cls2, s.order2, s.meta2, li, o3,
-                                                             m3, p.rerun_capped, p.rerun_cond, p.rerun_iters, skip, (float)p.w0); break;
-                case 1: k3_flag_class<4><<<fb, 256, 0, cs>>>(st32, sst, s.order, s.meta, p.flags, r, p.rerun_margin,
-                                                             p.rerun_pivot, wl, s.cls2, s.order2, s.meta2, li, o3,
-                                                             m3, p.rerun_capped, p.rerun_cond, p.rerun_iters, skip, (float)p.w0); break;
-                default: k3_flag_class<7><<<fb, 256, 0, cs>>>(st32, sst, s.order, s.meta, p.flags, r,
-                                                              p.rerun_margin, p.rerun_pivot, wl, s.cls2, s.order2,
-                                                              s.meta2, li, o3, m3, p.rerun_capped, p.rerun_cond, p.rerun_iters, skip, (float)p.w0); break;
-                }
-                if ((e = cudaGetLastError()) != cudaSuccess) return e;
-                bump();
-                K1Args k64 = k1;
-                // warm-started fits fall back to the reference start
-                if (p.warm) k64.init_params = nullptr;
-                k64.order = s.order2;
-                k64.meta = s.meta2;
-                k64.state = s.state64;
-                k64.pivot_thr = 0.0f;
-                k64.stats = s.stats + ST_N;  // counters of the re-run kept apart
-                if (long_q) {
-                    // the long re-runs: their own stream (when the chain has
-                    // one) and more threads per fit; launched first so that
-                    // in a serial call they start at the head
-                    K1Args kl = k64;
-                    kl.order = s.order3;
-                    kl.meta = s.meta3;
-                    cudaStream_t ls = cs;
-                    if (naux > 0 && p.aux_long[j]) {
-                        ls = p.aux_long[j];
-                        if ((e = cudaEventRecord(p.flagged[j], cs)) != cudaSuccess) return e;
-                        if ((e = cudaStreamWaitEvent(ls, p.flagged[j], 0)) != cudaSuccess) return e;
-                        used_long[j] = true;
-                    }
-                    e = launch_queues<double>(p, kl, cnt1, r_cap, tpb, false, p.long_rerun_threads_per_fit, ls,
-                                              err_detail);
-                    if (e != cudaSuccess) return e;
-                }
-                // the other flagged fits: fewer threads per fit, more fits in flight
-                e = launch_queues<double>(p, k64, cnt1, r_cap, tpb, false, p.rerun_threads_per_fit, cs, err_detail);
-            }
-        }
-        if (e != cudaSuccess) return e;
+        LOC_TRY(launch_team<double>(m, ta, r_most, n, p.blocks_per_sm, stream));
     }
-    for (int j = 0; j < naux; ++j) {
-        if (used[j]) {
-            if ((e = cudaEventRecord(p.join[j], p.aux[j])) != cudaSuccess) return e;
-            if ((e = cudaStreamWaitEvent(stream, p.join[j], 0)) != cudaSuccess) return e;
-        }
-        if (used_long[j]) {
-            if ((e = cudaEventRecord(p.join_long[j], p.aux_long[j])) != cudaSuccess) return e;
-            if ((e = cudaStreamWaitEvent(stream, p.join_long[j], 0)) != cudaSuccess) return e;
-        }
-    }
-    if (e != cudaSuccess) return e;
+#undef LOC_TRY
     mark(2);
     K2Args k2{(const Cand *)p.cands, n, p.method, p.w0, r_default,
               p.precision == 1 ? nullptr : (const float *)s.state,

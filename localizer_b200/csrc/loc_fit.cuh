@@ -30,7 +30,7 @@ struct Scratch {
     float *init;         // n * P: proposed starts (warm mode only)
 };
 
-constexpr int kMetaInts = 8 + 8 * (kMaxHalfWidth + 1);
+constexpr int kMetaInts = 8 + 6 * (kMaxHalfWidth + 1);
 
 struct FitParams {
     const uint16_t *frames;
@@ -73,9 +73,6 @@ struct FitParams {
     cudaStream_t aux[kMaxAux];  // optional auxiliary streams (NULL-terminated) for the class chains
     cudaEvent_t fork;           // fork / join events for them
     cudaEvent_t join[kMaxAux];
-    cudaStream_t aux_long[kMaxAux];  // optional streams for the long FP64 re-runs, one per chain
-    cudaEvent_t flagged[kMaxAux];    // chain j's flag pass done
-    cudaEvent_t join_long[kMaxAux];
     double *out;
     uint8_t *flags;
     // ROI mode (host-buffer calls): the pixels are not whole frames but the
