@@ -142,7 +142,7 @@ __global__ void k0_scatter(const int *cls, int n, int *meta, int *order)
 }
 
 // Appends i of the lanes with want to a list, one atomic per warp.
-__device__ __forceinline__ void push(bool want, int i, int *list, int *count)
+__device__ __forceinline__ void push(bool want, int i, int *list, int step, int *count)
 {
     const unsigned who = __ballot_sync(kFull, want);
     if (!who) return;
@@ -150,34 +150,50 @@ __device__ __forceinline__ void push(bool want, int i, int *list, int *count)
     int at = 0;
     if (lane == first) at = atomicAdd(count, __popc(who));
     at = __shfl_sync(kFull, at, first);
-    if (want) list[at + __popc(who & ((1u << lane) - 1))] = i;
+    if (want) list[(long long)(at + __popc(who & ((1u << lane) - 1))) * step] = i;
 }
 
 // Fits of the FP32 solver whose result could depend on its rounding go to an
 // FP64 re-run: a branch decision of the trust-region method was within
 // `margin` of its threshold, the undamped normal matrix had a pivot ratio
 // below `pivot` (ill-conditioned), the solver stopped for lack of progress, or
-// one of the options' rules holds. Walks the queue and appends them to order2
-// / meta2, or, when their FP32 solve took more than long_iters iterations and
-// a long queue exists, to order3 / meta3: the long fits set the length of the
-// re-run, so they are dequeued first.
+// one of the options' rules holds. Walks a list of fits (two lists, the
+// second backwards, for the suspended ones) and appends the flagged ones to
+// the short or, when their FP32 solve took more than long_iters iterations
+// and there is one, to the long FP64 list: the long fits set the length of the
+// re-run. Fits still suspended (cls2 kSuspended) are left for the pass over
+// them.
+constexpr int kSuspended = -2;
+struct FlagArgs {
+    const float *state32;
+    int stride;
+    const int *list, *count, *list_b, *count_b;   // list_b[-k]
+    const int *cls;
+    const uint8_t *flags;
+    int *cls2;
+    int suspended;       // the lists hold suspended fits (all finished by now)
+    int *shorts, *n_short, *longs, *n_long;       // entries at [k * step]; longs NULL: one list
+    int step;
+    float margin, pivot, cond, skip_rej, w0;
+    int warm_limit, long_iters, capped, iters_min;
+};
 template <int P>
-__global__ void k3_flag(const float *state32, int stride, const int *order, const int *meta, const int *cls,
-                        const uint8_t *flags, float margin, float pivot, int warm_limit, int *cls2,
-                        int *order2, int *meta2, int long_iters, int *order3, int *meta3, int capped,
-                        float cond, int iters_min, float skip_rej, float w0)
+__global__ void k3_flag(FlagArgs a)
 {
     using SL = StateLayout<P>;
     constexpr int IX = P == 5 ? 2 : P == 4 ? 1 : 3;
-    const int count = meta[M_TOTAL];
+    const int n_a = *a.count, count = n_a + (a.count_b ? *a.count_b : 0);
+    const float margin = a.margin, pivot = a.pivot, cond = a.cond, skip_rej = a.skip_rej, w0 = a.w0;
+    const int warm_limit = a.warm_limit, capped = a.capped, iters_min = a.iters_min;
     // whole warps walk together (push)
     for (int t0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); t0 < count; t0 += gridDim.x * blockDim.x) {
         const int t = t0 + (int)(threadIdx.x & 31);
-        const int i = t < count ? order[t] : 0;
-        const int r = t < count ? cls[i] : 0;
+        const int i = t >= count ? 0 : t < n_a ? a.list[t] : a.list_b[-(t - n_a)];
+        const int r = t < count ? a.cls[i] : 0;
         bool rerun = false, is_long = false;
-        if (t < count && flags[i] == F_PENDING) {
-            const float *s = state32 + (size_t)i * stride;
+        if (t < count && a.flags[i] == F_PENDING && (a.suspended || a.cls2[i] != kSuspended)) {
+            if (a.suspended) a.cls2[i] = -1;
+            const float *s = a.state32 + (size_t)i * a.stride;
             const float status = s[SL::STATUS];
             // warm-started fits (warm_limit > 0) that needed many iterations may
             // stop elsewhere than the reference start's trajectory would
@@ -217,13 +233,13 @@ __global__ void k3_flag(const float *state32, int stride, const int *order, cons
                 }
             }
             if (risky && !clear_reject) {
-                cls2[i] = r;
+                a.cls2[i] = r;
                 rerun = true;
-                is_long = meta3 && s[SL::ITERS] > (float)long_iters;
+                is_long = a.longs && s[SL::ITERS] > (float)a.long_iters;
             }
         }
-        push(rerun && !is_long, i, order2, &meta2[M_TOTAL]);
-        if (meta3) push(is_long, i, order3, &meta3[M_TOTAL]);
+        push(rerun && !is_long, i, a.shorts, a.step, a.n_short);
+        if (a.longs) push(is_long, i, a.longs, a.step, a.n_long);
     }
 }
 
@@ -247,8 +263,10 @@ struct K1Args {
     // list mode (r = 0): a list of candidates of any ROI size instead of one
     // class's part of the queue
     const int *list, *count;
+    int list_step;      // entry k at list[k * list_step]
     int *next;
     const int *cls;
+    int *mark;          // optional: suspended fits are marked here (cls2)
     int resume;         // the list's fits are suspended ones
     int least;          // lists of at most this many fits are left to the teams
     int budget;         // iterations a fit may use (0: all)
@@ -522,8 +540,9 @@ __device__ __forceinline__ void run_class(const K1Args &a, int r_class, int smem
             for (int k = 0; k < NT; ++k) o.A[k] = A[k];
             save_scalars<T>(o.sc, Scalars<T>{fnorm, delta, par, xnorm, minpiv_fit, margin_fit, it_state, iterations, xo,
                                              yo, TPF, esc_fit});
+            if (a.mark) a.mark[cidx] = kSuspended;
             if (over) a.cont[atomicAdd(a.n_cont, 1)] = cidx;
-            else a.left[atomicAdd(a.n_left, 1) * a.left_step] = cidx;
+            else a.left[(long long)atomicAdd(a.n_left, 1) * a.left_step] = cidx;
         }
     };
     // finish() and suspend() only mark the fit; its state is written at the
@@ -595,7 +614,7 @@ __device__ __forceinline__ void run_class(const K1Args &a, int r_class, int smem
             int my = -1;
             if (want) {
                 const int qi = base + __popc(need & ((1u << glead) - 1));
-                if (qi < ccount) my = queue[qi];
+                if (qi < ccount) my = queue[by_list ? (long long)qi * a.list_step : qi];
                 else exhausted = true;
             }
             int fr = 0;
@@ -1291,7 +1310,7 @@ cudaError_t launch_list_m(int m, const K1Args &ka, int r_cap, int tpb, int bps_r
 // Calls of at most this many candidates run on the team solver alone: that is
 // two fits for every warp of a full device (148 SMs x 12 warps). With one
 // thread per fit such a call leaves most of the device idle for as long as its
-// longest fit takes (1 200 ellipsoidal fits 550 us, by teams 300 us).
+// longest fit takes (200 symmetric fits 530 us, by teams 300 us).
 constexpr int kTeamOnlyFits = 3552;
 // Lists of at most this many fits go to the teams at once (FP32, FP64). FP32:
 // any value from 300 to 3552 measures the same; FP64: 3552 is the best of 1 to
@@ -1416,7 +1435,7 @@ cudaError_t enqueue_fit(const FitParams &p, const Scratch &s, cudaStream_t strea
     if (e != cudaSuccess) return e;
     if (rerun && (e = cudaMemsetAsync(s.meta2, 0, sizeof(int) * kMetaInts, stream)) != cudaSuccess) return e;
     const bool long_q = rerun && p.long_rerun_iters > 0;
-    if (long_q && (e = cudaMemsetAsync(s.meta3, 0, sizeof(int) * kMetaInts, stream)) != cudaSuccess) return e;
+    if (rerun && (e = cudaMemsetAsync(s.meta3, 0, sizeof(int) * kMetaInts, stream)) != cudaSuccess) return e;
     e = cudaMemsetAsync(s.stats, 0, sizeof(unsigned long long) * kStatWords, stream);
     if (e != cudaSuccess) return e;
     if (p.method == 6) {
@@ -1507,6 +1526,7 @@ cudaError_t enqueue_fit(const FitParams &p, const Scratch &s, cudaStream_t strea
     k1.init_params = p.warm ? s.init : p.init_params;
     k1.stats = s.stats;
     k1.cls = s.cls;
+    k1.list_step = 1;
     k1.cont = s.cont;
     k1.n_cont = s.meta + M_NCONT;
     k1.left = s.cont + n - 1;   // from the other end of the list: a fit is in one of the two
@@ -1571,6 +1591,7 @@ cudaError_t enqueue_fit(const FitParams &p, const Scratch &s, cudaStream_t strea
         K1Args kf = k1;
         kf.budget = two_level ? p.level0_budget : 0;
         kf.drain = p.threads_per_fit == 1 && m != 7 ? kDrain1 : 0;
+        kf.mark = rerun ? s.cls2 : nullptr;
         if ((e = fork()) != cudaSuccess) return e;
         int chain = 0;
         for (int r = r_most; r >= 1; --r) {
@@ -1591,65 +1612,114 @@ cudaError_t enqueue_fit(const FitParams &p, const Scratch &s, cudaStream_t strea
             kl.next = s.meta + M_CONTNEXT;
             kl.resume = 1;
             kl.least = kTeamFits32;
-            if ((e = side(0, &cs)) != cudaSuccess) return e;
+            if ((e = side(1, &cs)) != cudaSuccess) return e;
             LOC_TRY(launch_list_m<float>(m, kl, r_most, tpb, p.blocks_per_sm, p.tail_threads_per_fit, cs));
             ta.list[1] = TeamList{s.cont, s.meta + M_NCONT, 1, 0, 0, kTeamFits32};
         }
         ta.list[0] = left;
-        if ((e = side(1, &cs)) != cudaSuccess) return e;
+        if ((e = side(0, &cs)) != cudaSuccess) return e;
         LOC_TRY(launch_team<float>(m, ta, r_most, n, p.blocks_per_sm, cs));
-        if ((e = join()) != cudaSuccess) return e;
     }
     if (rerun) {
-        const int fb = n < 2 * 148 * 256 ? (n + 255) / 256 : 2 * 148;
-        const int wl = p.warm ? p.warm_iter_limit : 0;
-        const float *st32 = (const float *)s.state;
-        const int sst = state_stride(p.method);
-        int *o3 = long_q ? s.order3 : nullptr, *m3 = long_q ? s.meta3 : nullptr;
+        FlagArgs fa{};
+        fa.state32 = (const float *)s.state;
+        fa.stride = state_stride(p.method);
+        fa.cls = s.cls;
+        fa.flags = p.flags;
+        fa.cls2 = s.cls2;
+        fa.margin = p.rerun_margin;
+        fa.pivot = p.rerun_pivot;
+        fa.cond = p.rerun_cond;
         // a warm fit's reject says nothing about where the reference start's
         // path ends: with a proposal every flagged fit is re-run
-        const float skip = p.warm ? 0.0f : p.rerun_skip_rejected;
-        auto flag = [&](auto kern) {
-            kern<<<fb, 256, 0, stream>>>(st32, sst, s.order, s.meta, s.cls, p.flags, p.rerun_margin, p.rerun_pivot, wl,
-                                         s.cls2, s.order2, s.meta2, p.long_rerun_iters, o3, m3, p.rerun_capped,
-                                         p.rerun_cond, p.rerun_iters, skip, (float)p.w0);
+        fa.skip_rej = p.warm ? 0.0f : p.rerun_skip_rejected;
+        fa.w0 = (float)p.w0;
+        fa.warm_limit = p.warm ? p.warm_iter_limit : 0;
+        fa.long_iters = p.long_rerun_iters;
+        fa.capped = p.rerun_capped;
+        fa.iters_min = p.rerun_iters;
+        // One re-run: flag a set of fits and solve them again in FP64, on
+        // stream fs. Re-run 0 takes the fits that the first level finished (or
+        // all, in a team-only call) and runs beside the second level; re-run 1
+        // takes the fits that were suspended. Their lists share arrays from
+        // both ends and use different counters.
+        auto flag = [&](int set, cudaStream_t fs) -> cudaError_t {
+            FlagArgs f = fa;
+            f.list = set ? s.cont : s.order;
+            f.count = s.meta + (set ? M_NCONT : M_TOTAL);
+            f.list_b = set ? s.cont + n - 1 : nullptr;
+            f.count_b = set ? s.meta + M_NLEFT : nullptr;
+            f.suspended = set;
+            f.shorts = s.order2 + (set ? n - 1 : 0);
+            f.n_short = s.meta2 + (set ? M_NCONT : M_TOTAL);
+            f.longs = long_q ? s.order3 + (set ? n - 1 : 0) : nullptr;
+            f.n_long = s.meta3 + (set ? M_NCONT : M_TOTAL);
+            f.step = set ? -1 : 1;
+            const int fb = n < 2 * 148 * 256 ? (n + 255) / 256 : 2 * 148;
+            if (m == 0) k3_flag<5><<<fb, 256, 0, fs>>>(f);
+            else if (m == 1) k3_flag<4><<<fb, 256, 0, fs>>>(f);
+            else k3_flag<7><<<fb, 256, 0, fs>>>(f);
             return cudaGetLastError();
         };
-        LOC_TRY(m == 0 ? flag(k3_flag<5>) : m == 1 ? flag(k3_flag<4>) : flag(k3_flag<7>));
-        K1Args kd = k1;
-        kd.state = s.state64;
-        kd.stats = s.stats + ST_N;   // counters of the re-run kept apart
-        kd.pivot_thr = 0.0f;
-        if (p.warm) kd.init_params = nullptr;   // warm-started fits fall back to the reference start
-        kd.left = s.cont;                       // free again
-        kd.left_step = 1;
-        kd.n_left = s.meta2 + M_NLEFT;
-        kd.least = kTeamFits64;
-        ta.k = kd;
-        ta.switch_it = p.max_iter;
-        ta.next = s.meta2 + M_LEFTNEXT;
-        const int most = team_only ? n : kTeamFits64;
-        // the long re-runs first: they set the length of the launch
-        if (long_q) ta.list[0] = TeamList{s.order3, s.meta3 + M_TOTAL, 1, 1, p.long_rerun_threads_per_fit, most};
-        else ta.list[0] = TeamList{};
-        ta.list[1] = TeamList{s.order2, s.meta2 + M_TOTAL, 1, 1, p.rerun_threads_per_fit, most};
-        if (!team_only) {
-            // more flagged fits than the teams take: groups of threads first
-            if ((e = fork()) != cudaSuccess) return e;
-            for (int k = long_q ? 0 : 1; k < 2; ++k) {
-                const int tpf = k == 0 ? p.long_rerun_threads_per_fit : p.rerun_threads_per_fit;
-                kd.list = k == 0 ? s.order3 : s.order2;
-                kd.count = (k == 0 ? s.meta3 : s.meta2) + M_TOTAL;
-                kd.next = (k == 0 ? s.meta3 : s.meta2) + M_NEXT;
-                kd.drain = tpf <= 2 ? kDrain2 : 1;
-                if ((e = side(k, &cs)) != cudaSuccess) return e;
-                LOC_TRY(launch_list_m<double>(m, kd, r_most, tpb, p.blocks_per_sm, tpf, cs));
+        auto rerun_fits = [&](int set, cudaStream_t fs) -> cudaError_t {
+            const int step = set ? -1 : 1, c_total = set ? M_NCONT : M_TOTAL, c_next = set ? M_CONTNEXT : M_NEXT;
+            int *shorts = s.order2 + (set ? n - 1 : 0), *longs = long_q ? s.order3 + (set ? n - 1 : 0) : nullptr;
+            // the class order is used up: the fits left to the teams go there
+            int *left64 = s.order + (set ? n - 1 : 0);
+            int *meta_left = set ? s.meta3 : s.meta2;
+            K1Args kd = k1;
+            kd.state = s.state64;
+            kd.stats = s.stats + ST_N;   // counters of the re-run kept apart
+            kd.pivot_thr = 0.0f;
+            if (p.warm) kd.init_params = nullptr;   // warm-started fits fall back to the reference start
+            kd.left = left64;
+            kd.left_step = step;
+            kd.n_left = meta_left + M_NLEFT;
+            kd.least = kTeamFits64;
+            kd.list_step = step;
+            TeamArgs td{};
+            td.k = kd;
+            td.switch_it = p.max_iter;
+            td.q0 = td.q1 = 1;
+            td.next = meta_left + M_LEFTNEXT;
+            const int most = team_only ? n : kTeamFits64;
+            // the long re-runs first: they set the length of the launch
+            if (long_q) td.list[0] = TeamList{longs, s.meta3 + c_total, step, 1, p.long_rerun_threads_per_fit, most};
+            td.list[1] = TeamList{shorts, s.meta2 + c_total, step, 1, p.rerun_threads_per_fit, most};
+            if (!team_only) {
+                // more flagged fits than the teams take: groups of threads first
+                // (what the first level finished took at most its budget)
+                const bool no_long = !long_q || (set == 0 && two_level && p.level0_budget <= p.long_rerun_iters);
+                for (int k = no_long ? 1 : 0; k < 2; ++k) {
+                    const int tpf = k == 0 ? p.long_rerun_threads_per_fit : p.rerun_threads_per_fit;
+                    kd.list = k == 0 ? longs : shorts;
+                    kd.count = (k == 0 ? s.meta3 : s.meta2) + c_total;
+                    kd.next = (k == 0 ? s.meta3 : s.meta2) + c_next;
+                    kd.drain = tpf <= 2 ? kDrain2 : 1;
+                    LOC_TRY(launch_list_m<double>(m, kd, r_most, tpb, p.blocks_per_sm, tpf, fs));
+                }
+                td.list[2] = TeamList{left64, meta_left + M_NLEFT, step, 0, 0, n};
             }
-            if ((e = join()) != cudaSuccess) return e;
-            ta.list[2] = TeamList{s.cont, s.meta2 + M_NLEFT, 1, 0, 0, n};
+            LOC_TRY(launch_team<double>(m, td, r_most, n, p.blocks_per_sm, fs));
+            return cudaSuccess;
+        };
+        // flagged before the suspended ones: that pass gives their marks up
+        LOC_TRY(flag(0, stream));
+        if (!team_only) {
+            // the suspended fits' re-run follows both launches of the second level
+            if (naux > 0 && (e = cudaEventRecord(p.fork, stream)) != cudaSuccess) return e;
+            if ((e = side(0, &cs)) != cudaSuccess) return e;
+            if (naux > 0 && (e = cudaStreamWaitEvent(cs, p.fork, 0)) != cudaSuccess) return e;
+            if (naux > 1 && used[1]) {
+                if ((e = cudaEventRecord(p.join[1], p.aux[1])) != cudaSuccess) return e;
+                if ((e = cudaStreamWaitEvent(cs, p.join[1], 0)) != cudaSuccess) return e;
+            }
+            LOC_TRY(flag(1, cs));
+            if ((e = rerun_fits(1, cs)) != cudaSuccess) return e;
         }
-        LOC_TRY(launch_team<double>(m, ta, r_most, n, p.blocks_per_sm, stream));
+        if ((e = rerun_fits(0, stream)) != cudaSuccess) return e;
     }
+    if ((e = join()) != cudaSuccess) return e;
 #undef LOC_TRY
     mark(2);
     K2Args k2{(const Cand *)p.cands, n, p.method, p.w0, r_default,
