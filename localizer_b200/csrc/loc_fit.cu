@@ -682,19 +682,52 @@ __device__ __forceinline__ void run_class(const K1Args &a, int r_class, int smem
                 rbase = a.roi_slot ? (long long)a.roi_slot[my]
                                    : (long long)fr * a.frame_px + xo + (long long)yo * a.n_rows;
             }
-            // warp-cooperative ROI staging: global uint16 -> shared float
+            // warp-cooperative ROI staging: global uint16 -> shared float. The
+            // loads of up to four fits are issued before the first is stored:
+            // a trip refills about four of a warp's 32 fits, and one latency
+            // per fit and round was a quarter of the first level's time
+            // (520 000 dense fits: ellipsoidal 11.04 -> 10.47 ms, symmetric
+            // 6.88 -> 6.36 ms; fetching further queue entries into L2 ahead of
+            // time gave nothing more).
             unsigned got = __ballot_sync(kFull, my >= 0 && leader);
-            while (got) {
-                const int src = __ffs(got) - 1;
-                got &= got - 1;
-                const long long sbase = __shfl_sync(kFull, rbase, src);
-                const int side = S > 0 ? S : __shfl_sync(kFull, s, src);
-                const int pitch = a.roi_slot ? side : a.n_rows;   // a packed ROI's rows are 2r + 1 pixels apart
-                const uint16_t *fb = a.frames + sbase;
-                float *dst = smem + ((tid - lane + src) / TPF) * stride;
-                for (int k = lane; k < side * side; k += 32) {
-                    const int j = k / side, i = k - j * side;
-                    dst[k] = (float)__ldg(fb + i + (size_t)j * pitch);
+            if constexpr (S > 0) {
+                constexpr int N = (S * S + 31) / 32, G = 4;
+                while (got) {
+                    uint16_t px[G][N];
+                    int src[G];   // past the last fit, the last one again
+#pragma unroll
+                    for (int g = 0; g < G; ++g) {
+                        src[g] = got ? __ffs(got) - 1 : src[g > 0 ? g - 1 : 0];
+                        got &= got - 1;
+                        const uint16_t *fb = a.frames + __shfl_sync(kFull, rbase, src[g]);
+                        const int pitch = a.roi_slot ? S : a.n_rows;   // a packed ROI's rows are 2r + 1 pixels apart
+#pragma unroll
+                        for (int n = 0; n < N; ++n) {
+                            const int k = min(lane + 32 * n, S * S - 1), j = k / S, i = k - j * S;
+                            px[g][n] = __ldg(fb + i + (size_t)j * pitch);
+                        }
+                    }
+#pragma unroll
+                    for (int g = 0; g < G; ++g) {
+                        float *dst = smem + ((tid - lane + src[g]) / TPF) * stride;
+#pragma unroll
+                        for (int n = 0; n < N; ++n)
+                            if (lane + 32 * n < S * S) dst[lane + 32 * n] = (float)px[g][n];
+                    }
+                }
+            } else {
+                while (got) {
+                    const int src = __ffs(got) - 1;
+                    got &= got - 1;
+                    const long long sbase = __shfl_sync(kFull, rbase, src);
+                    const int side = __shfl_sync(kFull, s, src);
+                    const int pitch = a.roi_slot ? side : a.n_rows;
+                    const uint16_t *fb = a.frames + sbase;
+                    float *dst = smem + ((tid - lane + src) / TPF) * stride;
+                    for (int k = lane; k < side * side; k += 32) {
+                        const int j = k / side, i = k - j * side;
+                        dst[k] = (float)__ldg(fb + i + (size_t)j * pitch);
+                    }
                 }
             }
             __syncwarp();
