@@ -1355,19 +1355,40 @@ constexpr int kTeamFits32 = 3552, kTeamFits64 = 3552;
 // fits, while the symmetric ones lose 7.5 -> 7.8 ms without), the re-run with
 // two threads per fit, and FP64-precision calls.
 constexpr int kDrain1 = 4, kDrain2 = 3, kDrain64 = 8;
+// Lists of up to this many fits are solved by teams of four warps, longer ones
+// by teams of one. Four warps take 0.6 of the time per fit and the instructions
+// of nearly four, so they win while the longest fit sets the time: two (FP32)
+// and three (FP64) fits per resident block. Measured, one warp -> four: a frame
+// of 100 ellipsoidal fits 298 -> 248 us, 200 symmetric fits 362 -> 350 us, the
+// FP64 re-run of 262 of 520 000 symmetric fits 6.30 -> 5.70 ms for the call; with
+// 2 400 ellipsoidal re-runs 10.6 -> 11.8 ms, so they keep one warp.
+constexpr int kBlockFits32 = 1184, kBlockFits64 = 1332;
 
-template <int METHOD, typename T, bool ESC>
-cudaError_t launch_team_m(const TeamArgs &ta, int r_cap, int n_most, int bps_req, cudaStream_t stream)
+template <int METHOD, typename T, bool ESC, int W>
+cudaError_t launch_team_w(const TeamArgs &ta, int r_cap, int n_most, int bps_req, cudaStream_t stream)
 {
-    auto kern = k_team<METHOD, T, ESC>;
-    constexpr int tpb = 128, per_block = tpb / 32;
-    const int smem = per_block * team_smem<METHOD, T>(r_cap);
+    auto kern = k_team<METHOD, T, ESC, W>;
+    constexpr int tpb = 128, per_block = tpb / 32 / W;
+    const int smem = per_block * team_smem<METHOD, T, W>(r_cap);
     int grid = 0;
     const cudaError_t e = persistent_grid(kern, tpb, smem, bps_req, &grid);
     if (e != cudaSuccess) return e;
     const int blocks = (n_most + per_block - 1) / per_block;
     kern<<<blocks < grid ? blocks : grid, tpb, smem, stream>>>(ta, r_cap);
     return cudaGetLastError();
+}
+
+template <int METHOD, typename T, bool ESC>
+cudaError_t launch_team_m(TeamArgs ta, int r_cap, int n_most, int bps_req, cudaStream_t stream)
+{
+    const int line = sizeof(T) == 8 ? kBlockFits64 : kBlockFits32;
+    ta.over = 0;
+    ta.upto = line;
+    cudaError_t e = launch_team_w<METHOD, T, ESC, 4>(ta, r_cap, n_most < line ? n_most : line, bps_req, stream);
+    if (e != cudaSuccess || n_most <= line) return e;
+    ta.over = line;
+    ta.upto = n_most;
+    return launch_team_w<METHOD, T, ESC, 1>(ta, r_cap, n_most, bps_req, stream);
 }
 
 // One team launch (method m of the solver) over at most n_most fits.

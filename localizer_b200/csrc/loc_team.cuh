@@ -1,4 +1,4 @@
-// Team solver: a warp works on one fit.
+// Team solver: a warp, or a block of four warps, works on one fit.
 //
 // The thread-per-fit solver (run_class in loc_fit.cu) has the better
 // throughput while every lane has a fit, but a single fit takes as long as
@@ -21,6 +21,10 @@
 //      threads' butterfly.
 // The damped solve runs on every lane (its chain of pivots is serial); the
 // per-parameter work of the accept/reject logic is spread over the lanes.
+//
+// In a team of four warps the pass is spread over 128 threads, and every warp
+// does the rest of the iteration for itself: all of them read the same sums and
+// arrive at the same step, so nothing has to be handed round.
 #pragma once
 
 #include "loc_device.cuh"
@@ -45,7 +49,14 @@ __device__ __forceinline__ void lds_pair(double2 &v, uint32_t at)
     asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "r"(at));
 }
 
-constexpr int kTeamChunk = 64;   // pixels whose columns are in shared memory at a time
+constexpr int kTeamChunk = 64;   // pixels per warp of the team whose columns are in shared memory at a time
+
+// a team is a warp (W == 1) or a block of W warps
+template <int W> __device__ __forceinline__ void team_sync()
+{
+    if constexpr (W == 1) __syncwarp();
+    else __syncthreads();
+}
 
 // Columns of one pixel, in pairs: the Jacobian columns, 1, r (and a zero to
 // fill the pair), then del and 2 r - del.
@@ -305,11 +316,11 @@ template <typename T> struct PixelEval<7, T> {
 // then the state: A and v of the current and of the trial point, the scaled
 // matrix, and per-parameter vectors.
 __host__ __device__ constexpr int team_roi_bytes(int r) { return ((2 * r + 1) * (2 * r + 1) * 4 + 15) / 16 * 16; }
-template <int METHOD, typename T> __host__ __device__ constexpr int team_smem(int r_cap)
+template <int METHOD, typename T, int W> __host__ __device__ constexpr int team_smem(int r_cap)
 {
     using D = TeamDims<METHOD>;
-    return team_roi_bytes(r_cap) + (kTeamChunk * D::VS + 8 * D::NB * 4) * (int)sizeof(T) +
-           ((2 * D::NE + D::NT + 3 * 8) * (int)sizeof(T) + 15) / 16 * 16;
+    return team_roi_bytes(r_cap) + (W * kTeamChunk * D::VS + 8 * D::NB * 4) * (int)sizeof(T) +
+           ((2 * D::NE + W * (D::NT + 3 * 8)) * (int)sizeof(T) + 4 + 15) / 16 * 16;
 }
 
 // largest of the (non-negative) values of lanes 0 to 7
@@ -334,24 +345,25 @@ __device__ __forceinline__ double max_of_8(double v)
 // over consecutive records whatever q_n is. Units (a 2 x 2 block of one
 // partial sum) are dealt to the lanes in rounds; their sums rest in shared
 // memory between chunks.
-template <int METHOD, typename T>
+template <int METHOD, typename T, int W>
 __device__ __forceinline__ bool team_pass(const float *roi, int s, T *chunk, T *sums, T *res,
                                        const T (&te)[Traits<METHOD>::P], const T (&dt)[Traits<METHOD>::P],
-                                       const int (&entry)[TeamDims<METHOD>::NE / 32 + 1], long long unit, T w0, T inv_s2,
-                                       int q_n, int wide, int lane)
+                                       const int (&entry)[TeamDims<METHOD>::NE / (32 * W) + 1], long long unit, T w0, T inv_s2,
+                                       int q_n, int wide, int tl)
 {
     using D = TeamDims<METHOD>;
     using V2 = typename Vec2<T>::type;
     constexpr int NV = 2 * (D::PAIRS + 1);
     PixelEval<METHOD, T> px;
-    px.prep(te, dt, w0, lane, row_fuse_square<T>(s, q_n));
+    px.prep(te, dt, w0, threadIdx.x & 31, row_fuse_square<T>(s, q_n));
     // columns per partial sum; the first `more` have one more
     const int qmask = q_n - 1, qshift = q_n == 8 ? 3 : q_n >> 1;
     const int units = D::NB * q_n, per = s >> qshift, more = s & qmask;
-    const int rows = kTeamChunk / s;
+    constexpr int TN = 32 * W;
+    const int rows = W * kTeamChunk / s;
     const uint32_t chunk_at = (uint32_t)__cvta_generic_to_shared(chunk);
-    // this lane's pixels of a chunk: lane and lane + 32
-    const int ja = lane / s, ia = lane - ja * s, jb = (lane + 32) / s, ib = lane + 32 - jb * s;
+    // this thread's pixels of a chunk: tl and tl + TN
+    const int ja = tl / s, ia = tl - ja * s, jb = (tl + TN) / s, ib = tl + TN - jb * s;
     T dqmax = T(0);
     for (int j0 = 0; j0 < s; j0 += rows) {
         const int nr = min(rows, s - j0), n = nr * s;
@@ -369,12 +381,12 @@ __device__ __forceinline__ bool team_pass(const float *roi, int s, T *chunk, T *
                 dst[v] = w;
             }
         };
-        if (lane < n) {
+        if (tl < n) {
             // both evaluations side by side: the second hides the first's latency
-            const bool two = lane + 32 < n;
+            const bool two = tl + TN < n;
             T oa[NV], ob[NV];
-            const T da = px.eval(ia, j0 + ja, (T)roi[j0 * s + lane], oa);
-            const T db = px.eval(ib, j0 + jb, (T)roi[j0 * s + (two ? lane + 32 : lane)], ob);
+            const T da = px.eval(ia, j0 + ja, (T)roi[j0 * s + tl], oa);
+            const T db = px.eval(ib, j0 + jb, (T)roi[j0 * s + (two ? tl + TN : tl)], ob);
             dqmax = fmax(dqmax, da);
             put(place(ia, ja), oa);
             if (two) {
@@ -382,15 +394,15 @@ __device__ __forceinline__ bool team_pass(const float *roi, int s, T *chunk, T *
                 put(place(ib, jb), ob);
             }
         }
-        __syncwarp();
+        team_sync<W>();
 #pragma unroll 1
-        for (int k = 0; k * 32 + lane < units; ++k) {
+        for (int k = 0; k * TN + tl < units; ++k) {
             const int w = (int)(unit >> (k * 11)), q = (w >> 8) & 7;   // k < 3 only: NB * 8 <= 96
             constexpr uint32_t kRec = D::VS * sizeof(T), kPair = sizeof(V2);
             const uint32_t p = chunk_at + nr * (q * per + min(q, more)) * kRec;
             uint32_t pa = p + (w & 15) * kPair, pb = p + ((w >> 4) & 15) * kPair;
             const int cnt = nr * (per + (q < more ? 1 : 0));
-            V2 *sum = reinterpret_cast<V2 *>(sums + (k * 32 + lane) * 4);
+            V2 *sum = reinterpret_cast<V2 *>(sums + (k * TN + tl) * 4);
             V2 lo = sum[0], hi = sum[1];
             if (j0 == 0) lo.x = lo.y = hi.x = hi.y = T(0);
             // operands are read four records ahead (past the last record they
@@ -425,12 +437,12 @@ __device__ __forceinline__ bool team_pass(const float *roi, int s, T *chunk, T *
             sum[0] = lo;
             sum[1] = hi;
         }
-        __syncwarp();   // the sums are complete; the next chunk may overwrite this one
+        team_sync<W>();   // the sums are complete; the next chunk may overwrite this one
     }
     // the partial sums in the order of the threads' butterfly
 #pragma unroll
-    for (int k = 0; k < D::NE / 32 + 1; ++k) {
-        const int e = lane + k * 32;
+    for (int k = 0; k < D::NE / TN + 1; ++k) {
+        const int e = tl + k * TN;
         if (e >= D::NE) break;
         const T *p = sums + entry[k];
         auto at = [&](int q) { return p[q * D::NB * 4]; };
@@ -445,6 +457,7 @@ __device__ __forceinline__ bool team_pass(const float *roi, int s, T *chunk, T *
         }
         res[e] = e < D::NT + D::P ? v * inv_s2 : v;
     }
+    if constexpr (W > 1) return __syncthreads_and(dqmax < T(0.25)) != 0;
     __syncwarp();
     return __ballot_sync(kFull, !(dqmax < T(0.25))) == 0;
 }
@@ -464,9 +477,10 @@ struct TeamArgs {
     TeamList list[3];
     int *next;              // dequeue cursor over the lists
     int q0, q1, switch_it;  // partial sums up to and from iteration switch_it
+    int over, upto;         // works only when the lists hold more than `over` and at most `upto` fits
 };
 
-template <int METHOD, typename T, bool ESC>
+template <int METHOD, typename T, bool ESC, int W>
 __global__ void __launch_bounds__(128, sizeof(T) == 8 || ESC ? 3 : 4) k_team(TeamArgs a, int r_cap)
 {
     using D = TeamDims<METHOD>;
@@ -474,14 +488,17 @@ __global__ void __launch_bounds__(128, sizeof(T) == 8 || ESC ? 3 : 4) k_team(Tea
     using SL = StateLayout<P>;
     extern __shared__ __align__(16) unsigned char sm_team[];
     const K1Args &ka = a.k;
-    const int lane = threadIdx.x & 31;
-    unsigned char *base = sm_team + (threadIdx.x / 32) * team_smem<METHOD, T>(r_cap);
+    constexpr int TN = 32 * W;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x / 32;
+    const int tl = W == 1 ? lane : threadIdx.x;      // thread of the team
+    unsigned char *base = sm_team + (W == 1 ? warp : 0) * team_smem<METHOD, T, W>(r_cap);
     float *roi = reinterpret_cast<float *>(base);
     T *chunk = reinterpret_cast<T *>(base + team_roi_bytes(r_cap));
-    T *sums = chunk + kTeamChunk * D::VS;
+    T *sums = chunk + W * kTeamChunk * D::VS;
     T *buf0 = sums + 8 * D::NB * 4;            // A, v, |r|^2 and its change, for two points
-    T *msv = buf0 + 2 * D::NE;
+    T *msv = buf0 + 2 * D::NE + (W == 1 ? 0 : warp) * (NT + 3 * 8);   // each warp's own
     T *s_inv = msv + NT, *s_te = s_inv + 8, *s_dt = s_te + 8;
+    int *s_next = reinterpret_cast<int *>(buf0 + 2 * D::NE + W * (NT + 3 * 8));
     const T inv_s2 = sizeof(T) == 4 ? (T)ka.inv_s2 : (T)ka.inv_s2_d;
     const T inv_abs_s = sizeof(T) == 4 ? (T)ka.inv_abs_s : (T)ka.inv_abs_s_d;
     const T w0 = (T)ka.w0;
@@ -492,18 +509,19 @@ __global__ void __launch_bounds__(128, sizeof(T) == 8 || ESC ? 3 : 4) k_team(Tea
         if (n <= a.list[k].most) n_all += n;
         ends[k] = n_all;
     }
+    if (n_all <= a.over || n_all > a.upto) return;
     unsigned st[ST_N];
 #pragma unroll
     for (int k = 0; k < ST_N; ++k) st[k] = 0;
     // lane k < P: parameter k; everything else is the same on every lane
     const bool mine = lane < P;
     const int own = mine ? lane : 0;
-    int entry[D::NE / 32 + 1];
+    int entry[D::NE / TN + 1];
 #pragma unroll
-    for (int k = 0; k < D::NE / 32 + 1; ++k) entry[k] = lane + k * 32 < D::NE ? team_entry<METHOD>(lane + k * 32) : 0;
-    // this lane's units of a pass, 11 bits each, and its entry of the scaled matrix
-    const long long unit = (long long)team_unit<METHOD>(lane) | (long long)team_unit<METHOD>(lane + 32) << 11 |
-                           (long long)team_unit<METHOD>(lane + 64) << 22;
+    for (int k = 0; k < D::NE / TN + 1; ++k) entry[k] = tl + k * TN < D::NE ? team_entry<METHOD>(tl + k * TN) : 0;
+    // this thread's units of a pass, 11 bits each, and its lane's entry of the scaled matrix
+    const long long unit = (long long)team_unit<METHOD>(tl) | (long long)team_unit<METHOD>(tl + TN) << 11 |
+                           (long long)team_unit<METHOD>(tl + 2 * TN) << 22;
     int mi = 0, mj = lane;
     while (mj >= P - mi && mi < P) {
         mj -= P - mi;
@@ -516,8 +534,14 @@ __global__ void __launch_bounds__(128, sizeof(T) == 8 || ESC ? 3 : 4) k_team(Tea
     while (true) {
         // ---- next fit ----
         int qi = 0;
-        if (lane == 0) qi = atomicAdd(a.next, 1);
-        qi = __shfl_sync(kFull, qi, 0);
+        if (tl == 0) qi = atomicAdd(a.next, 1);
+        if constexpr (W == 1) {
+            qi = __shfl_sync(kFull, qi, 0);
+        } else {
+            if (tl == 0) *s_next = qi;
+            __syncthreads();
+            qi = *s_next;
+        }
         if (qi >= n_all) break;
         int li = 0;
         while (qi >= ends[li]) ++li;
@@ -531,11 +555,11 @@ __global__ void __launch_bounds__(128, sizeof(T) == 8 || ESC ? 3 : 4) k_team(Tea
                                               : (long long)cd.frame * ka.frame_px + xo + (long long)yo * ka.n_rows;
             const int pitch = ka.roi_slot ? s : ka.n_rows;   // a packed ROI's rows are 2r + 1 pixels apart
             const uint16_t *fb = ka.frames + org;
-            int j = lane / s, i = lane - j * s;
+            int j = tl / s, i = tl - j * s;
 #pragma unroll 4
-            for (int k = lane; k < npx; k += 32) {
+            for (int k = tl; k < npx; k += TN) {
                 roi[k] = (float)__ldg(fb + i + (size_t)j * pitch);
-                i += 32;
+                i += TN;
                 while (i >= s) {
                     i -= s;
                     ++j;
@@ -566,9 +590,9 @@ __global__ void __launch_bounds__(128, sizeof(T) == 8 || ESC ? 3 : 4) k_team(Tea
                 th = o.th[lane];
                 sc = o.D[lane];
                 dx = o.dx[lane];
-                cur[NT + lane] = o.v[lane];
+                if (W == 1 || warp == 0) cur[NT + lane] = o.v[lane];
             }
-            for (int k = lane; k < NT; k += 32) cur[k] = o.A[k];
+            for (int k = tl; k < NT; k += TN) cur[k] = o.A[k];
             const Scalars<T> c = load_scalars<T>(o.sc);
             fnorm = c.fnorm;
             delta = c.delta;
@@ -581,7 +605,7 @@ __global__ void __launch_bounds__(128, sizeof(T) == 8 || ESC ? 3 : 4) k_team(Tea
             esc_fit = c.esc;
             if (sizeof(T) == 8) q_fix = c.q_n;
         }
-        __syncwarp();
+        team_sync<W>();
         auto theta_abs = [&](T t) -> T { return lane == IX ? t + (T)xo : (lane == IX + 1 ? t + (T)yo : t); };
         // largest step / test_delta tolerance over the parameters (at t), and
         // whether every step is below its tolerance
@@ -627,7 +651,7 @@ __global__ void __launch_bounds__(128, sizeof(T) == 8 || ESC ? 3 : 4) k_team(Tea
                 T npiv;
                 lmpar_scaled<P, T, ESC, false>(Ms, gv, inv_dv, sym_fuse(s, q_n), delta, par, z, ka.pivot_thr, nl, ne, sing,
                                                npiv, margin_fit);
-                if (lane == 0) {
+                if (tl == 0) {
                     st[ST_LAMBDA] += nl;
                     st[ST_ESC] += ne;
                 }
@@ -676,9 +700,9 @@ __global__ void __launch_bounds__(128, sizeof(T) == 8 || ESC ? 3 : 4) k_team(Tea
                 tev[k] = s_te[k];
                 dtv[k] = s_dt[k];
             }
-            const bool near = team_pass<METHOD, T>(roi, s, chunk, sums, alt, tev, dtv, entry, unit, w0, inv_s2, q_n,
-                                                   ka.compensated, lane);
-            if (lane == 0) {
+            const bool near = team_pass<METHOD, T, W>(roi, s, chunk, sums, alt, tev, dtv, entry, unit, w0, inv_s2, q_n,
+                                                      ka.compensated, tl);
+            if (tl == 0) {
                 if (first) {
                     st[ST_J] += 1;
                     st[ST_PIXJ] += npx;
@@ -753,7 +777,7 @@ __global__ void __launch_bounds__(128, sizeof(T) == 8 || ESC ? 3 : 4) k_team(Tea
                     first = false;
                 } else {
                     ++it_state;
-                    if (lane == 0) {
+                    if (tl == 0) {
                         st[ST_J] += 1;   // the accepted trial's Jacobian
                         st[ST_PIXJ] += npx;
                     }
@@ -780,9 +804,9 @@ __global__ void __launch_bounds__(128, sizeof(T) == 8 || ESC ? 3 : 4) k_team(Tea
         bool small;
         const T lastr = step_test(th, small);
         T *o = (T *)ka.state + (size_t)cidx * ka.state_stride;
-        if (mine) o[lane] = th;
-        for (int k = lane; k < NT; k += 32) o[P + k] = cur[k];
-        if (lane == 0) {
+        if (tl < P) o[lane] = th;
+        for (int k = tl; k < NT; k += TN) o[P + k] = cur[k];
+        if (tl == 0) {
             o[SL::FNORM] = fnorm;
             o[SL::ITERS] = (T)iterations;
             o[SL::STATUS] = (T)done;
@@ -795,9 +819,9 @@ __global__ void __launch_bounds__(128, sizeof(T) == 8 || ESC ? 3 : 4) k_team(Tea
             st[ST_FITS] += 1;
             st[ST_ITERS] += iterations;
         }
-        __syncwarp();   // the next fit's ROI and sums take this one's place
+        team_sync<W>();   // the next fit's ROI and sums take this one's place
     }
-    if (lane == 0) {
+    if (tl == 0) {
         const unsigned long long all = (unsigned long long)(clock64() - t_begin);
         st[ST_CYC_STEP] += (unsigned)((all - c_pass) >> 10);
         st[ST_CYC_PASS] += (unsigned)(c_pass >> 10);
