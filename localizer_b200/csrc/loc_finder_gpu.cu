@@ -151,17 +151,31 @@ __global__ void __launch_bounds__(32 * kWarps) k_glrt_fast(const uint16_t *frame
     __syncthreads();
     const int c = (int)c_min;
     unsigned sum = 0;
-    for (int ty = warp; ty < FT::ROWS; ty += kWarps) {
-        const int yy = ty0 - HALF + ty;
-        const bool row_ok = yy >= 0 && yy < p.n_cols;
-        const bool inner = ty >= HALF && ty < HALF + FT::TH;
-        const uint16_t *rp = fr + (long long)yy * p.n_rows;
-        for (int tx = lane; tx < FT::PITCH; tx += 32) {
-            const int xx = tx0 - HALF + tx;
-            const bool ok = row_ok && xx >= 0 && xx < p.n_rows;
-            const int v = ok ? (int)rp[xx] : c;
-            tile[ty * FT::PITCH + tx] = (float)(v - c);
-            if (ok && inner && tx >= HALF && tx < HALF + FT::TW) sum += (unsigned)v;
+    // all loads of two rows before the first store: with one load at a time the
+    // tile's memory latencies were a third of the kernel (500 frames of 512 x 512:
+    // search 1.26 -> 0.81 ms; four rows at a time measure the same)
+    constexpr int NX = (FT::PITCH + 31) / 32, NR = 2;
+    for (int tr = warp * NR; tr < FT::ROWS; tr += kWarps * NR) {
+        uint16_t px[NR][NX];
+#pragma unroll
+        for (int u = 0; u < NR; ++u) {
+            const uint16_t *rp = fr + (size_t)min(max(ty0 - HALF + tr + u, 0), p.n_cols - 1) * p.n_rows;
+#pragma unroll
+            for (int n = 0; n < NX; ++n) px[u][n] = rp[min(max(tx0 - HALF + lane + 32 * n, 0), p.n_rows - 1)];
+        }
+#pragma unroll
+        for (int u = 0; u < NR; ++u) {
+            const int ty = tr + u, yy = ty0 - HALF + ty;
+            if (ty >= FT::ROWS) break;
+            const bool row_ok = yy >= 0 && yy < p.n_cols;
+            const bool inner = ty >= HALF && ty < HALF + FT::TH;
+#pragma unroll
+            for (int n = 0; n < NX; ++n) {
+                const int tx = lane + 32 * n, xx = tx0 - HALF + tx;
+                const bool ok = row_ok && xx >= 0 && xx < p.n_rows;
+                if (tx < FT::PITCH) tile[ty * FT::PITCH + tx] = ok ? (float)((int)px[u][n] - c) : 0.f;
+                if (ok && inner && tx >= HALF && tx < HALF + FT::TW) sum += px[u][n];
+            }
         }
     }
     add_total(sum, &total[f]);
