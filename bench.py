@@ -218,7 +218,7 @@ def make_workload(w):
     assign_half_widths(w, cands)
     finder = {"ms": f_ms, "frames_per_s": w.n_frames / (f_ms / 1e3), "candidates": int(n),
               "frame_read_gbs": frames_dev.numel() * 2 / (f_ms / 1e3) / 1e9,
-              "kernels": "k_glrt, k_union, k_flatten, k_count_roots, k_assign, k_accumulate, k_emit"}
+              "kernels": "k_glrt_fast, k_group, k_offsets, k_place"}
     log(f"[bench] {w.n_frames} frames rendered in {t1 - t0:.1f}s, {len(cands)} candidates found on the GPU in "
         f"{f_ms:.1f} ms")
     return frames_dev, cands, finder
@@ -768,8 +768,8 @@ def main():
                              "no ncu capture of the current solver chain",
                              "peak_source": "nominal FP32 (148 SM x 128 lanes x 2 x max SM clock); "
                                             "no measured FP32 peak in MEASURED_PEAKS.json",
-                             "kernel": "k1_lm_fit + k3_flag_class + k2_finalize (plain arm, every ROI class and "
-                                       "level)", "kernel_ms": k_ms, "flops_per_step": flops,
+                             "kernel": "k1_lm_fit + k_team + k3_flag + k2_finalize (plain arm, every ROI class "
+                                       "and level)", "kernel_ms": k_ms, "flops_per_step": flops,
                              "kernel_ms_source": "step device time (method calls overlap)" if concurrent else
                              "solver stage events of the call"},
                 "finder": finder, "stats": st, "clocks": clocks, "e2e": e2e, "cpu_baseline": cpu,
@@ -872,7 +872,7 @@ def measure_next_rows(L, torch, eng, frames_dev, frames_host, part, w0, rows_pla
     torch.cuda.synchronize()
     ms = a.elapsed_time(b) / reps
     gbs = src.numel() * 6 / (ms / 1e3) / 1e9
-    out["ingest"] = {"kernel": "k_ingest_rm<float>", "frames": nf, "ms_per_call": ms, "frames_per_s": nf / (ms / 1e3),
+    out["ingest"] = {"kernel": "k_ingest_rm_even<float>", "frames": nf, "ms_per_call": ms, "frames_per_s": nf / (ms / 1e3),
                      "achieved_gbs": gbs, "peak_gbs": hbm_peak, "frac": gbs / hbm_peak,
                      "bytes_per_pixel": 6, "check": "lossless round trip of the uint16 stack",
                      "timing": "per call, including the call's host synchronisation for the lossy count",

@@ -109,9 +109,9 @@ typedef struct loc_options {
     int32_t blocks_per_sm;     /* 0: occupancy maximum */
     int32_t stage_u16;         /* reserved, ignored: ROIs are staged in shared
                                   memory as FP32 (kept for the struct layout) */
-    int32_t max_half_width;    /* 0: the solver reads the largest ROI half-width
-                                  present back from the device (one small
-                                  synchronous copy); > 0: caller guarantees
+    int32_t max_half_width;    /* 0: a call too large for the team solver reads
+                                  the largest ROI half-width present back from
+                                  the device (one small synchronous copy); > 0: caller guarantees
                                   every candidate's r is at most this (no host
                                   synchronisation, capturable in a CUDA graph);
                                   larger candidates are flagged LOC_FLAG_BAD_INPUT */
@@ -167,8 +167,8 @@ typedef struct loc_options {
     int32_t long_rerun_iters;  /* FP64 re-runs of fits whose FP32 solve took more
                                   iterations than this form their own queue,
                                   solved with long_rerun_threads_per_fit threads
-                                  per fit on a second stream of their chain (they
-                                  set the length of the re-run); 0: default, the
+                                  per fit ahead of the short ones (they set the
+                                  length of the re-run); 0: default, the
                                   level-0 budget; < 0: one queue */
     int32_t long_rerun_threads_per_fit; /* 1, 2, 4 or 8; 0: default 8 */
     int32_t compensated;       /* 1: two-level summation of the FP32 normal

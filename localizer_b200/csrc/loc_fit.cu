@@ -7,7 +7,11 @@
 //      idle lanes from the queue with one atomic and stages their ROIs from
 //      the HBM-resident uint16 frames with warp-cooperative loads into shared
 //      memory; every loop trip is one model/Jacobian/normal-equation pass
-//      for all active lanes (see loc_device.cuh).
+//      for all active lanes (see loc_device.cuh). Level 0 solves fresh fits
+//      per ROI side, level 1 (8 threads per fit) a list of suspended ones; the
+//      FP64 re-run walks lists as well.
+//   team (loc_team.cuh) — a warp or a block per fit, where latency counts.
+//   K3 flag — which FP32 fits are re-run in FP64.
 //   K2 finalize — FP64: covariance (J^T J)^-1, uncertainty scaling, the
 //      reference's accept/reject rules and output columns.
 #include "loc_device.cuh"
@@ -1343,7 +1347,7 @@ cudaError_t launch_list_m(int m, const K1Args &ka, int r_cap, int tpb, int bps_r
 // Calls of at most this many candidates run on the team solver alone: that is
 // two fits for every warp of a full device (148 SMs x 12 warps). With one
 // thread per fit such a call leaves most of the device idle for as long as its
-// longest fit takes (200 symmetric fits 530 us, by teams 300 us).
+// longest fit takes (160 symmetric fits 530 us, by teams 300 us).
 constexpr int kTeamOnlyFits = 3552;
 // Lists of at most this many fits go to the teams at once (FP32, FP64). FP32:
 // any value from 300 to 3552 measures the same; FP64: 3552 is the best of 1 to
@@ -1351,7 +1355,7 @@ constexpr int kTeamOnlyFits = 3552;
 constexpr int kTeamFits32 = 3552, kTeamFits64 = 3552;
 // A warp that has run dry hands its last fits over at this many groups or
 // fewer: FP32 with one thread per fit (the ellipsoidal models, whose fits
-// differ most in length, keep them: measured 11.9 against 12.6 ms at 336 000
+// differ most in length, keep them: measured 11.9 against 12.6 ms at 520 000
 // fits, while the symmetric ones lose 7.5 -> 7.8 ms without), the re-run with
 // two threads per fit, and FP64-precision calls.
 constexpr int kDrain1 = 4, kDrain2 = 3, kDrain64 = 8;
@@ -1359,7 +1363,7 @@ constexpr int kDrain1 = 4, kDrain2 = 3, kDrain64 = 8;
 // by teams of one. Four warps take 0.6 of the time per fit and the instructions
 // of nearly four, so they win while the longest fit sets the time: two (FP32)
 // and three (FP64) fits per resident block. Measured, one warp -> four: a frame
-// of 100 ellipsoidal fits 298 -> 248 us, 200 symmetric fits 362 -> 350 us, the
+// of 80 ellipsoidal fits 298 -> 248 us, 160 symmetric fits 362 -> 350 us, the
 // FP64 re-run of 262 of 520 000 symmetric fits 6.30 -> 5.70 ms for the call; with
 // 2 400 ellipsoidal re-runs 10.6 -> 11.8 ms, so they keep one warp.
 constexpr int kBlockFits32 = 1184, kBlockFits64 = 1332;

@@ -97,7 +97,7 @@ __device__ __forceinline__ double objective(double x0, double y0, double sd, dou
     for (int k0 = 0; k0 < roi.npx; k0 += kChunk) {
         __syncwarp();   // the previous chunk's terms have been read
         // one copy in the code: with two side by side the instruction fetches
-        // cost more than the overlap gave (21 000 fits: 15.0 -> 13.9 ms)
+        // cost more than the overlap gave (16 800 fits: 15.0 -> 13.7 ms)
 #pragma unroll 1
         for (int u = 0; u < 2; ++u) {
             const int k = k0 + u * 32 + lane;
