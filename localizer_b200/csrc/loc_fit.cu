@@ -1243,11 +1243,13 @@ __global__ void k2_finalize(K2Args a)
 
 int solver_method(int method) { return method == 5 ? 7 : method; }
 
-// Blocks of a persistent kernel: every SM filled to its occupancy.
+// Blocks of a persistent kernel: every SM filled to its occupancy. The limit
+// on its shared memory is set to the device's, whatever this launch needs: host
+// threads with other ROI sizes launch the same kernels.
 template <typename F>
 cudaError_t persistent_grid(F *kern, int tpb, int smem, int bps_req, int *grid)
 {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     if (e != cudaSuccess) return e;
     int dev = 0, nsm = 0, bps = 0;
     cudaGetDevice(&dev);

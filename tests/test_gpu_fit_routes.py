@@ -92,3 +92,32 @@ def test_options_on_both_routes(engine, kw):
     r, f = _fit(engine, frames, cands[:900], 7, **kw)
     np.testing.assert_array_equal(f, flags[:900])
     np.testing.assert_array_equal(r, rows[:900])
+
+
+def test_threads_with_other_sizes():
+    """Two host threads, each with its own engine, fit ROIs of the smallest and
+    the largest size at the same time: the launches share their kernels."""
+    import threading
+    work = {half: _stack(half, n, half) for half, n in ((2, 4200), (16, 700))}
+    want, got, errors = {}, {}, []
+    engines = {half: L.Engine(0) for half in work}
+    for half, (frames, cands) in work.items():
+        want[half] = _fit(engines[half], frames, cands, 7)
+
+    def run(half):
+        try:
+            for _ in range(20):
+                got[half] = _fit(engines[half], *work[half], 7)
+        except Exception as e:   # shown by the main thread
+            errors.append((half, e))
+
+    threads = [threading.Thread(target=run, args=(half,)) for half in work]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors
+    for half in work:
+        np.testing.assert_array_equal(got[half][1], want[half][1])
+        np.testing.assert_array_equal(got[half][0], want[half][0])
+        engines[half].close()
