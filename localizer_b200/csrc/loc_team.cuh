@@ -39,17 +39,22 @@ template <> struct Vec2<double> { using type = double2; };
 // One pair from shared memory, kept where it stands in the program: the chains
 // below read their operands ahead, and left to itself the compiler moves the
 // loads back to their use (20 000 all-FP64 fits 2.36 ms, with this 2.19 ms;
-// the FP32 calls stay within 3 %).
+// the FP32 calls stay within 3 %). The memory clobber orders the loads after
+// the plain stores that filled the records.
 __device__ __forceinline__ void lds_pair(float2 &v, uint32_t at)
 {
-    asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(at));
+    asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(at) : "memory");
 }
 __device__ __forceinline__ void lds_pair(double2 &v, uint32_t at)
 {
-    asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "r"(at));
+    asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "r"(at) : "memory");
 }
 
 constexpr int kTeamChunk = 64;   // pixels per warp of the team whose columns are in shared memory at a time
+constexpr int kTeamAhead = 4;    // records that a chain reads ahead, past the chunk's last one too
+// records of a team's chunk: what is read ahead of a full chunk lies in memory
+// that nobody writes
+__host__ __device__ constexpr int team_records(int warps) { return warps * kTeamChunk + kTeamAhead; }
 
 // a team is a warp (W == 1) or a block of W warps
 template <int W> __device__ __forceinline__ void team_sync()
@@ -319,7 +324,7 @@ __host__ __device__ constexpr int team_roi_bytes(int r) { return ((2 * r + 1) * 
 template <int METHOD, typename T, int W> __host__ __device__ constexpr int team_smem(int r_cap)
 {
     using D = TeamDims<METHOD>;
-    return team_roi_bytes(r_cap) + (W * kTeamChunk * D::VS + 8 * D::NB * 4) * (int)sizeof(T) +
+    return team_roi_bytes(r_cap) + (team_records(W) * D::VS + 8 * D::NB * 4) * (int)sizeof(T) +
            ((2 * D::NE + W * (D::NT + 3 * 8)) * (int)sizeof(T) + 4 + 15) / 16 * 16;
 }
 
@@ -405,11 +410,12 @@ __device__ __forceinline__ bool team_pass(const float *roi, int s, T *chunk, T *
             V2 *sum = reinterpret_cast<V2 *>(sums + (k * TN + tl) * 4);
             V2 lo = sum[0], hi = sum[1];
             if (j0 == 0) lo.x = lo.y = hi.x = hi.y = T(0);
-            // operands are read four records ahead (past the last record they
-            // come from whatever follows and are not used)
-            V2 x[4], y[4];
+            // operands are read kTeamAhead records ahead (past the last record
+            // they come from another partial sum's, or from the room behind
+            // the chunk, and are not used)
+            V2 x[kTeamAhead], y[kTeamAhead];
 #pragma unroll
-            for (int d = 0; d < 4; ++d) {
+            for (int d = 0; d < kTeamAhead; ++d) {
                 lds_pair(x[d], pa + d * kRec);
                 lds_pair(y[d], pb + d * kRec);
             }
@@ -419,18 +425,18 @@ __device__ __forceinline__ bool team_pass(const float *roi, int s, T *chunk, T *
                 hi.x = fma(x[d].y, y[d].x, hi.x);
                 hi.y = fma(x[d].y, y[d].y, hi.y);
             };
-            int at = 4;
-            for (; at <= cnt; at += 4) {
-                pa += 4 * kRec;
-                pb += 4 * kRec;
+            int at = kTeamAhead;
+            for (; at <= cnt; at += kTeamAhead) {
+                pa += kTeamAhead * kRec;
+                pb += kTeamAhead * kRec;
 #pragma unroll
-                for (int d = 0; d < 4; ++d) {
+                for (int d = 0; d < kTeamAhead; ++d) {
                     step(d);
                     lds_pair(x[d], pa + d * kRec);
                     lds_pair(y[d], pb + d * kRec);
                 }
             }
-            const int rest = cnt - at + 4;
+            const int rest = cnt - at + kTeamAhead;
             if (rest > 0) step(0);
             if (rest > 1) step(1);
             if (rest > 2) step(2);
@@ -494,7 +500,7 @@ __global__ void __launch_bounds__(128, sizeof(T) == 8 || ESC ? 3 : 4) k_team(Tea
     unsigned char *base = sm_team + (W == 1 ? warp : 0) * team_smem<METHOD, T, W>(r_cap);
     float *roi = reinterpret_cast<float *>(base);
     T *chunk = reinterpret_cast<T *>(base + team_roi_bytes(r_cap));
-    T *sums = chunk + W * kTeamChunk * D::VS;
+    T *sums = chunk + team_records(W) * D::VS;
     T *buf0 = sums + 8 * D::NB * 4;            // A, v, |r|^2 and its change, for two points
     T *msv = buf0 + 2 * D::NE + (W == 1 ? 0 : warp) * (NT + 3 * 8);   // each warp's own
     T *s_inv = msv + NT, *s_te = s_inv + 8, *s_dt = s_te + 8;
