@@ -385,13 +385,13 @@ __global__ void __launch_bounds__(32 * kWarps, 4) k_mlewg(MlArgs a)
         return;
     }
     const int s = 2 * r + 1;
-    // Localization.cpp:694-704
-    const int xo = (int)floor(c.x - (double)r), yo = (int)floor(c.y - (double)r);
-    const int xm = xo + s - 1, ym = yo + s - 1;
-    if (xo < 0 || xm > a.n_rows - 1 || yo < 0 || ym > a.n_cols - 1) {
+    // Localization.cpp:694-704; in double, as a position far outside does not fit an int
+    const double xod = floor(c.x - (double)r), yod = floor(c.y - (double)r);
+    if (xod < 0 || xod + 2 * r > a.n_rows - 1 || yod < 0 || yod + 2 * r > a.n_cols - 1) {
         reject(1);
         return;
     }
+    const int xo = (int)xod, yo = (int)yod, xm = xo + s - 1, ym = yo + s - 1;
     const int npx = s * s, room = smem_px(a.r_cap);
     unsigned char *mine = sm + warp * smem_per_fit(a.r_cap);
     double *term = reinterpret_cast<double *>(mine), *lg = term + kChunk;
