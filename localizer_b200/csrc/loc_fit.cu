@@ -1743,13 +1743,17 @@ cudaError_t enqueue_fit(const FitParams &p, const Scratch &s, cudaStream_t strea
             td.q0 = td.q1 = 1;
             td.next = meta_left + M_LEFTNEXT;
             const int most = team_only ? n : kTeamFits64;
+            // No thread groups for the long re-runs of set 0: what the first
+            // level finished took at most its budget, but for fits whose residual
+            // became exactly zero (they end at the iteration cap at once, see
+            // start_iteration). Those go to the teams, however many they are.
+            const bool no_long = !long_q || (set == 0 && two_level && p.level0_budget <= p.long_rerun_iters);
             // the long re-runs first: they set the length of the launch
-            if (long_q) td.list[0] = TeamList{longs, s.meta3 + c_total, step, 1, p.long_rerun_threads_per_fit, most};
+            if (long_q)
+                td.list[0] = TeamList{longs, s.meta3 + c_total, step, 1, p.long_rerun_threads_per_fit, no_long ? n : most};
             td.list[1] = TeamList{shorts, s.meta2 + c_total, step, 1, p.rerun_threads_per_fit, most};
             if (!team_only) {
                 // more flagged fits than the teams take: groups of threads first
-                // (what the first level finished took at most its budget)
-                const bool no_long = !long_q || (set == 0 && two_level && p.level0_budget <= p.long_rerun_iters);
                 for (int k = no_long ? 1 : 0; k < 2; ++k) {
                     const int tpf = k == 0 ? p.long_rerun_threads_per_fit : p.rerun_threads_per_fit;
                     kd.list = k == 0 ? longs : shorts;
