@@ -1370,31 +1370,18 @@ constexpr int kDrain1 = 4, kDrain2 = 3, kDrain64 = 8;
 // 2 400 ellipsoidal re-runs 10.6 -> 11.8 ms, so they keep one warp.
 constexpr int kBlockFits32 = 1184, kBlockFits64 = 1332;
 
-template <int METHOD, typename T, bool ESC, int W>
-cudaError_t launch_team_w(const TeamArgs &ta, int r_cap, int n_most, int bps_req, cudaStream_t stream)
+template <int METHOD, typename T, bool ESC>
+cudaError_t launch_team_m(const TeamArgs &ta, int r_cap, int n_most, int bps_req, cudaStream_t stream)
 {
-    auto kern = k_team<METHOD, T, ESC, W>;
-    constexpr int tpb = 128, per_block = tpb / 32 / W;
-    const int smem = per_block * team_smem<METHOD, T, W>(r_cap);
+    auto kern = k_team<METHOD, T, ESC>;
+    constexpr int tpb = 128, line = sizeof(T) == 8 ? kBlockFits64 : kBlockFits32;
+    const int one = team_smem<METHOD, T, 4>(r_cap), four = 4 * team_smem<METHOD, T, 1>(r_cap);
+    const int smem = one > four ? one : four;
     int grid = 0;
     const cudaError_t e = persistent_grid(kern, tpb, smem, bps_req, &grid);
     if (e != cudaSuccess) return e;
-    const int blocks = (n_most + per_block - 1) / per_block;
-    kern<<<blocks < grid ? blocks : grid, tpb, smem, stream>>>(ta, r_cap);
+    kern<<<n_most < grid ? n_most : grid, tpb, smem, stream>>>(ta, r_cap, line);
     return cudaGetLastError();
-}
-
-template <int METHOD, typename T, bool ESC>
-cudaError_t launch_team_m(TeamArgs ta, int r_cap, int n_most, int bps_req, cudaStream_t stream)
-{
-    const int line = sizeof(T) == 8 ? kBlockFits64 : kBlockFits32;
-    ta.over = 0;
-    ta.upto = line;
-    cudaError_t e = launch_team_w<METHOD, T, ESC, 4>(ta, r_cap, n_most < line ? n_most : line, bps_req, stream);
-    if (e != cudaSuccess || n_most <= line) return e;
-    ta.over = line;
-    ta.upto = n_most;
-    return launch_team_w<METHOD, T, ESC, 1>(ta, r_cap, n_most, bps_req, stream);
 }
 
 // One team launch (method m of the solver) over at most n_most fits.

@@ -483,16 +483,17 @@ struct TeamArgs {
     TeamList list[3];
     int *next;              // dequeue cursor over the lists
     int q0, q1, switch_it;  // partial sums up to and from iteration switch_it
-    int over, upto;         // works only when the lists hold more than `over` and at most `upto` fits
 };
 
+// The fits of the lists (n_all of them, list k up to ends[k]), by teams of W
+// warps.
 template <int METHOD, typename T, bool ESC, int W>
-__global__ void __launch_bounds__(128, sizeof(T) == 8 || ESC ? 3 : 4) k_team(TeamArgs a, int r_cap)
+__device__ __forceinline__ void team_fits(const TeamArgs &a, int r_cap, int n_all, const int (&ends)[3],
+                                          unsigned char *sm_team)
 {
     using D = TeamDims<METHOD>;
     constexpr int P = D::P, NT = D::NT, IX = Traits<METHOD>::IX;
     using SL = StateLayout<P>;
-    extern __shared__ __align__(16) unsigned char sm_team[];
     const K1Args &ka = a.k;
     constexpr int TN = 32 * W;
     const int lane = threadIdx.x & 31, warp = threadIdx.x / 32;
@@ -508,14 +509,6 @@ __global__ void __launch_bounds__(128, sizeof(T) == 8 || ESC ? 3 : 4) k_team(Tea
     const T inv_s2 = sizeof(T) == 4 ? (T)ka.inv_s2 : (T)ka.inv_s2_d;
     const T inv_abs_s = sizeof(T) == 4 ? (T)ka.inv_abs_s : (T)ka.inv_abs_s_d;
     const T w0 = (T)ka.w0;
-    int ends[3], n_all = 0;
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        const int n = a.list[k].count ? *a.list[k].count : 0;
-        if (n <= a.list[k].most) n_all += n;
-        ends[k] = n_all;
-    }
-    if (n_all <= a.over || n_all > a.upto) return;
     unsigned st[ST_N];
 #pragma unroll
     for (int k = 0; k < ST_N; ++k) st[k] = 0;
@@ -835,6 +828,27 @@ __global__ void __launch_bounds__(128, sizeof(T) == 8 || ESC ? 3 : 4) k_team(Tea
         for (int k = 0; k < ST_N; ++k)
             if (st[k]) atomicAdd(&ka.stats[k], (unsigned long long)st[k]);
     }
+}
+
+// Lists of up to `line` fits are solved by teams of four warps, longer ones by
+// teams of one (kBlockFits32, kBlockFits64): the length is known on the device
+// only. One launch that holds both takes 5 to 8 us less than two of which one
+// returns at once, in the chain of every call beyond the warps alone (12 000
+// fixed-width fits of 5 x 5 ROIs: 144 -> 137 us).
+template <int METHOD, typename T, bool ESC>
+__global__ void __launch_bounds__(128, sizeof(T) == 8 || ESC ? 3 : 4) k_team(TeamArgs a, int r_cap, int line)
+{
+    extern __shared__ __align__(16) unsigned char sm_team[];
+    int ends[3], n_all = 0;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const int n = a.list[k].count ? *a.list[k].count : 0;
+        if (n <= a.list[k].most) n_all += n;
+        ends[k] = n_all;
+    }
+    if (n_all == 0) return;
+    if (n_all <= line) team_fits<METHOD, T, ESC, 4>(a, r_cap, n_all, ends, sm_team);
+    else team_fits<METHOD, T, ESC, 1>(a, r_cap, n_all, ends, sm_team);
 }
 
 }  // namespace
