@@ -1361,6 +1361,14 @@ constexpr int kTeamFits32 = 3552, kTeamFits64 = 3552;
 // fits, while the symmetric ones lose 7.5 -> 7.8 ms without), the re-run with
 // two threads per fit, and FP64-precision calls.
 constexpr int kDrain1 = 4, kDrain2 = 3, kDrain64 = 8;
+// Calls whose ROIs are all 3 x 3: a thread is through with nine pixels sooner
+// than a team with its sums and barriers, so the groups keep their fits and
+// only lists of a length that leaves the device idle go to the teams. 20 000
+// fits, with the lines above -> these: FP64 ellipsoidal 6.8 -> 4.1 ms,
+// symmetric 3.0 -> 2.5 ms; FP32 ellipsoidal 4.7 -> 4.1 ms, symmetric 4.3 -> 3.4
+// ms. From 5 x 5 ROIs on the lines above win (FP64 ellipsoidal 1.9 against
+// 3.1 ms).
+constexpr int kTeamFitsTiny = 300;
 // Lists of up to this many fits are solved by teams of four warps, longer ones
 // by teams of one. Four warps take 0.6 of the time per fit and the instructions
 // of nearly four, so they win while the longest fit sets the time: two (FP32)
@@ -1610,6 +1618,8 @@ cudaError_t enqueue_fit(const FitParams &p, const Scratch &s, cudaStream_t strea
     };
 #define LOC_TRY(call) do { if ((e = (call)) != cudaSuccess) { if (e == cudaErrorInvalidValue) *err_detail = 1; return e; } bump(); } while (0)
     cudaStream_t cs;
+    const bool tiny = r_most == 1;   // 3 x 3 ROIs only
+    const int fits32 = tiny ? kTeamFitsTiny : kTeamFits32, fits64 = tiny ? kTeamFitsTiny : kTeamFits64;
     const bool fp64 = p.precision == 1;
     const bool two_level = !fp64 && p.level0_budget > 0 && p.level0_budget < p.max_iter;
     TeamArgs ta{};
@@ -1629,7 +1639,7 @@ cudaError_t enqueue_fit(const FitParams &p, const Scratch &s, cudaStream_t strea
         kf.list = s.order;
         kf.count = s.meta + M_TOTAL;
         kf.next = s.meta + M_NEXT;
-        kf.drain = kDrain64;
+        kf.drain = tiny ? 0 : kDrain64;
         LOC_TRY(launch_list_m<double>(m, kf, r_most, tpb, p.blocks_per_sm, 1, stream));
         ta.list[0] = left;
         LOC_TRY(launch_team<double>(m, ta, r_most, n, p.blocks_per_sm, stream));
@@ -1637,7 +1647,7 @@ cudaError_t enqueue_fit(const FitParams &p, const Scratch &s, cudaStream_t strea
         // first level: the fresh candidates, one launch per ROI class
         K1Args kf = k1;
         kf.budget = two_level ? p.level0_budget : 0;
-        kf.drain = p.threads_per_fit == 1 && m != 7 ? kDrain1 : 0;
+        kf.drain = p.threads_per_fit == 1 && m != 7 && !tiny ? kDrain1 : 0;
         kf.mark = rerun ? s.cls2 : nullptr;
         if ((e = fork()) != cudaSuccess) return e;
         int chain = 0;
@@ -1658,10 +1668,10 @@ cudaError_t enqueue_fit(const FitParams &p, const Scratch &s, cudaStream_t strea
             kl.count = s.meta + M_NCONT;
             kl.next = s.meta + M_CONTNEXT;
             kl.resume = 1;
-            kl.least = kTeamFits32;
+            kl.least = fits32;
             if ((e = side(1, &cs)) != cudaSuccess) return e;
             LOC_TRY(launch_list_m<float>(m, kl, r_most, tpb, p.blocks_per_sm, p.tail_threads_per_fit, cs));
-            ta.list[1] = TeamList{s.cont, s.meta + M_NCONT, 1, 0, 0, kTeamFits32};
+            ta.list[1] = TeamList{s.cont, s.meta + M_NCONT, 1, 0, 0, fits32};
         }
         ta.list[0] = left;
         if ((e = side(0, &cs)) != cudaSuccess) return e;
@@ -1722,14 +1732,14 @@ cudaError_t enqueue_fit(const FitParams &p, const Scratch &s, cudaStream_t strea
             kd.left = left64;
             kd.left_step = step;
             kd.n_left = meta_left + M_NLEFT;
-            kd.least = kTeamFits64;
+            kd.least = fits64;
             kd.list_step = step;
             TeamArgs td{};
             td.k = kd;
             td.switch_it = p.max_iter;
             td.q0 = td.q1 = 1;
             td.next = meta_left + M_LEFTNEXT;
-            const int most = team_only ? n : kTeamFits64;
+            const int most = team_only ? n : fits64;
             // No thread groups for the long re-runs of set 0: what the first
             // level finished took at most its budget, but for fits whose residual
             // became exactly zero (they end at the iteration cap at once, see
@@ -1746,7 +1756,7 @@ cudaError_t enqueue_fit(const FitParams &p, const Scratch &s, cudaStream_t strea
                     kd.list = k == 0 ? longs : shorts;
                     kd.count = (k == 0 ? s.meta3 : s.meta2) + c_total;
                     kd.next = (k == 0 ? s.meta3 : s.meta2) + c_next;
-                    kd.drain = tpf <= 2 ? kDrain2 : 1;
+                    kd.drain = tiny ? 0 : tpf <= 2 ? kDrain2 : 1;
                     LOC_TRY(launch_list_m<double>(m, kd, r_most, tpb, p.blocks_per_sm, tpf, fs));
                 }
                 td.list[2] = TeamList{left64, meta_left + M_NLEFT, step, 0, 0, n};

@@ -37,14 +37,17 @@ def _fit(engine, frames, cands, method, **kw):
 @pytest.mark.parametrize("method,half,budget,long_iters,tail,short,long_,serial", [
     (7, 4, 3, 0, 8, 2, 8, 0), (7, 5, 2, 12, 4, 1, 4, 0), (7, 3, 4, 2, 1, 4, 2, 0), (7, 6, 3, -1, 8, 8, 8, 1),
     (0, 4, 3, 0, 8, 2, 8, 0), (0, 5, 2, 8, 4, 4, 1, 0), (0, 3, 6, 3, 8, 8, 4, 1), (0, 7, 4, -1, 1, 1, 8, 0),
-    (1, 4, 2, 0, 8, 2, 8, 0), (1, 2, 3, 2, 4, 4, 2, 1), (5, 4, 3, 6, 8, 2, 4, 0)])
+    (1, 4, 2, 0, 8, 2, 8, 0), (1, 2, 3, 2, 4, 4, 2, 1), (5, 4, 3, 6, 8, 2, 4, 0), (7, 1, 3, 0, 8, 2, 8, 0),
+    (0, 1, 4, 12, 4, 1, 4, 0), (1, 1, 3, 0, 8, 2, 8, 0)])
 def test_long_lists(method, half, budget, long_iters, tail, short, long_, serial):
     frames, cands = _stack(half, N, 31 * half + method)
     kw = dict(level0_budget=budget, long_rerun_iters=long_iters, tail_threads_per_fit=tail,
               rerun_threads_per_fit=short, long_rerun_threads_per_fit=long_)
     eng = L.Engine(0)
     whole = _fit(eng, frames, cands, method, serial_classes=serial, **kw)
-    assert eng.stats()["fits_fp64_rerun"] > 2 * TEAM_ONLY   # all but the fits that FP32 left at the iteration cap
+    # all but the fits that FP32 left at the iteration cap, which of five
+    # parameters in nine pixels are most (3 x 3 ROIs have a lower line)
+    assert eng.stats()["fits_fp64_rerun"] > (TEAM_ONLY if half == 1 else 2 * TEAM_ONLY)
     again = _fit(eng, frames, cands, method, serial_classes=serial, **kw)
     parts = [_fit(eng, frames, cands[k:k + PART], method, **kw) for k in range(0, N, PART)]
     eng.close()
