@@ -129,6 +129,9 @@ template <typename T, int N> struct StateArr<T, N, true> {
 // products that must round on their own, whatever they feed
 __device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
 __device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+// sums of a rounded product (not to be fused with it)
+__device__ __forceinline__ float add_rn(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ double add_rn(double a, double b) { return __dadd_rn(a, b); }
 
 // sum += x^2 for the terms i = 0, 1, ... (x0: the first): FP32 fuses every
 // term with the sum before it; FP64 fuses the first term with the rounded
@@ -196,24 +199,42 @@ __device__ __forceinline__ T expm1_series(T y)
     return y * p;
 }
 
-// Which product of the row term -dxs^2 - dys (2 w + dys) of pass_sym and
-// pass_fixed is fused with the other, rounded one: the square (true) or the
-// second. They differ in the last bit; each ROI side and group size has always
-// had the one given here, and every solver of a fit has to use it.
-template <typename T> __host__ __device__ constexpr bool row_fuse_square(int side, int threads)
+// Roundings of the symmetric and fixed-width models that depend on the ROI side
+// and the threads per fit. They differ in the last bit; every size has always
+// had the one given here (the compiler's choice in a kernel per side and group
+// size), and a fit that changes solver on its way needs the same in all of
+// them, so they are written out. Sides 5 to 17 had kernels of their own, with
+// 1, 4 and 8 threads, the others and the FP64 pivot escalation (ESC) one for
+// all sides.
+template <bool ESC> __host__ __device__ constexpr bool own_kernel(int side, int threads)
 {
-    return threads > 1 && (sizeof(T) == 8 || side < 9 || side > 17);
+    return !ESC && side >= 5 && side <= 17 && threads <= 8;
 }
-template <typename T> __device__ __forceinline__ T row_term(int side, int threads, T dxs, T dys, T wy)
+// The row term -dxs^2 - dys (2 w + dys) of pass_sym and pass_fixed: the second
+// product fused with the rounded first (true), or both rounded.
+template <int METHOD, typename T, bool ESC> __host__ __device__ constexpr bool row_fused(int side, int threads)
 {
-    const T t2 = fma(T(2), wy, dys);
-    return row_fuse_square<T>(side, threads) ? fma(-dxs, dxs, -mul_rn(dys, t2)) : fma(-dys, t2, -mul_rn(dxs, dxs));
+    return threads == 1 || threads == 16 ? true
+         : sizeof(T) == 8 ? false
+         : own_kernel<ESC>(side, threads) ? threads == 4 || side >= 9 : ESC && METHOD == 0;
+}
+template <typename T> __device__ __forceinline__ T row_term(bool fused, T dxs, T dys, T wy)
+{
+    const T t2 = fma(T(2), wy, dys), sq = mul_rn(dxs, dxs);
+    return fused ? fma(-dys, t2, -sq) : -sq - mul_rn(dys, t2);
+}
+// The FP32 symmetric solve: whether its forward substitution takes the
+// unrounded product (see chol_solve), bit 0 for the undamped solve, bit 1 for
+// the damped ones.
+template <bool ESC> __host__ __device__ constexpr int sym_fuse(int side, int threads)
+{
+    return own_kernel<ESC>(side, threads) && (threads == 1 ? side == 5 : side <= 13) ? 0 : 3;
 }
 
 // S > 0: compile-time ROI side (rows fully unrolled); S == 0: runtime side s_rt.
 template <int S, int TPF, typename T>
-__device__ __forceinline__ void pass_sym(const float *__restrict__ roi, int ld, int s_rt, int q, const T (&th)[5],
-                                         const T (&dth)[5], T (&acc)[14], T (&vv)[5], T &chi2, T &dchi, T &dqmax)
+__device__ __forceinline__ void pass_sym(const float *__restrict__ roi, int ld, int s_rt, int q, bool fused,
+                                         const T (&th)[5], const T (&dth)[5], T (&acc)[14], T (&vv)[5], T &chi2, T &dchi, T &dqmax)
 {
     const int s = S > 0 ? S : s_rt;
     const T A = th[0], w = th[1], x0 = th[2], y0 = th[3], b = th[4];
@@ -254,9 +275,9 @@ __device__ __forceinline__ void pass_sym(const float *__restrict__ roi, int ld, 
         acc[0] = fma(e, e, acc[0]);   acc[1] = fma(e, jr, acc[1]);   acc[2] = fma(e, jx, acc[2]);
         acc[3] = fma(e, jy, acc[3]);  acc[4] += e;
         acc[5] = fma(jr, jr, acc[5]); acc[6] = fma(jr, jx, acc[6]); acc[7] = fma(jr, jy, acc[7]);
-        acc[8] += jr;
-        acc[9] = fma(jx, jx, acc[9]); acc[10] = fma(jx, jy, acc[10]); acc[11] += jx;
-        acc[12] = fma(jy, jy, acc[12]); acc[13] += jy;
+        acc[8] = add_rn(acc[8], jr);
+        acc[9] = fma(jx, jx, acc[9]); acc[10] = fma(jx, jy, acc[10]); acc[11] = add_rn(acc[11], jx);
+        acc[12] = fma(jy, jy, acc[12]); acc[13] = add_rn(acc[13], jy);
         vv[0] = fma(e, r, vv[0]); vv[1] = fma(jr, r, vv[1]); vv[2] = fma(jx, r, vv[2]);
         vv[3] = fma(jy, r, vv[3]); vv[4] += r;
         chi2 = fma(r, r, chi2);
@@ -268,14 +289,14 @@ __device__ __forceinline__ void pass_sym(const float *__restrict__ roi, int ld, 
         for (int k = q; k < s * s; k += TPF) {
             const int j = k / s, i = k - j * s;
             const T wy = (T)j - y0;
-            body(i, wy, wy * wy, -dxs * dxs - dys * (T(2) * wy + dys), roi + j * s * ld);
+            body(i, wy, wy * wy, row_term<T>(fused, dxs, dys, wy), roi + j * s * ld);
         }
     } else {
 #pragma unroll 1
     for (int j = 0; j < s; ++j) {
         const T wy = (T)j - y0;
         const T wy2 = wy * wy;
-        const T krow = S > 0 || TPF > 8 ? -dxs * dxs - dys * (T(2) * wy + dys) : row_term<T>(s, TPF, dxs, dys, wy);  // (d2' - d2) minus its u term
+        const T krow = row_term<T>(fused, dxs, dys, wy);  // (d2' - d2) minus its u term
         const float *row = roi + j * s * ld;
         if (S > 0) {
             // two columns per trip: unrolling all of them made the per-class
@@ -294,7 +315,7 @@ __device__ __forceinline__ void pass_sym(const float *__restrict__ roi, int ld, 
 }
 
 template <int S, int TPF, typename T>
-__device__ __forceinline__ void pass_fixed(const float *__restrict__ roi, int ld, int s_rt, int q, T w0,
+__device__ __forceinline__ void pass_fixed(const float *__restrict__ roi, int ld, int s_rt, int q, bool fused, T w0,
                                            const T (&th)[4],
                                            const T (&dth)[4], T (&acc)[9], T (&vv)[4], T &chi2, T &dchi, T &dqmax)
 {
@@ -327,8 +348,8 @@ __device__ __forceinline__ void pass_fixed(const float *__restrict__ roi, int ld
         const T ex = e * ka_x;
         const T jx = u * ex, jy = wy * ex;
         acc[0] = fma(e, e, acc[0]); acc[1] = fma(e, jx, acc[1]); acc[2] = fma(e, jy, acc[2]); acc[3] += e;
-        acc[4] = fma(jx, jx, acc[4]); acc[5] = fma(jx, jy, acc[5]); acc[6] += jx;
-        acc[7] = fma(jy, jy, acc[7]); acc[8] += jy;
+        acc[4] = fma(jx, jx, acc[4]); acc[5] = fma(jx, jy, acc[5]); acc[6] = add_rn(acc[6], jx);
+        acc[7] = fma(jy, jy, acc[7]); acc[8] = add_rn(acc[8], jy);
         vv[0] = fma(e, r, vv[0]); vv[1] = fma(jx, r, vv[1]); vv[2] = fma(jy, r, vv[2]); vv[3] += r;
         chi2 = fma(r, r, chi2);
     };
@@ -337,14 +358,14 @@ __device__ __forceinline__ void pass_fixed(const float *__restrict__ roi, int ld
         for (int k = q; k < s * s; k += TPF) {
             const int j = k / s, i = k - j * s;
             const T wy = (T)j - y0;
-            body(i, wy, wy * wy, -dxs * dxs - dys * (T(2) * wy + dys), roi + j * s * ld);
+            body(i, wy, wy * wy, row_term<T>(fused, dxs, dys, wy), roi + j * s * ld);
         }
     } else {
 #pragma unroll 1
     for (int j = 0; j < s; ++j) {
         const T wy = (T)j - y0;
         const T wy2 = wy * wy;
-        const T krow = S > 0 || TPF > 8 ? -dxs * dxs - dys * (T(2) * wy + dys) : row_term<T>(s, TPF, dxs, dys, wy);
+        const T krow = row_term<T>(fused, dxs, dys, wy);
         const float *row = roi + j * s * ld;
         if (S > 0) {
             // two columns per trip: unrolling all of them made the per-class
@@ -427,7 +448,7 @@ __device__ __forceinline__ void pass_ell(const float *__restrict__ roi, int ld, 
         for (int m = 0; m < 6; ++m) {
 #pragma unroll
             for (int n = m; n < 6; ++n) acc[o + n - m] = fma(col[m], col[n], acc[o + n - m]);
-            acc[o + 6 - m] += col[m];
+            acc[o + 6 - m] = add_rn(acc[o + 6 - m], col[m]);
             o += 7 - m;
         }
 #pragma unroll
@@ -479,18 +500,6 @@ __device__ __forceinline__ void pass_ell(const float *__restrict__ roi, int ld, 
         }
     }
     }
-}
-
-// Which of two roundings the FP32 symmetric solve uses in its forward
-// substitution, by ROI side and threads per fit: bit 0 for the undamped
-// solve, bit 1 for the damped ones. The two differ in the last bit of the
-// step; a size has always had the one given here, and every solver of a fit
-// has to use it for the fit's path to be the same in all of them.
-__host__ __device__ constexpr int sym_fuse(int side, int threads)
-{
-    return threads == 1 ? (side == 5 ? 0 : 3)
-         : threads != 8 ? 0
-         : (side >= 9 && side <= 13) || side == 7 || side == 5 ? 0 : 3;
 }
 
 // ---------------------------------------------------------------------------
@@ -572,9 +581,9 @@ __device__ __forceinline__ int chol_solve(const MA &Ms, MS par, const MS (&v)[P]
             if (k > ii) sacc -= L[pkl(k, ii)] * zz[k];
         zz[ii] = sacc * inv[ii];
     }
-    T n2 = T(0);
+    T n2 = T(0), zz0;
 #pragma unroll
-    for (int i = 0; i < P; ++i) n2 += zz[i] * zz[i];
+    for (int i = 0; i < P; ++i) add_square<T>(zz[i], i, zz0, n2);
     const T zn = fsqrt(n2);
     T q2 = T(0);
     if (zn > T(0)) {

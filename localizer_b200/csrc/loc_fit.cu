@@ -287,22 +287,24 @@ struct K1Args {
 
 template <int METHOD, int S, int TPF, typename T> struct Pass;
 template <int S, int TPF, typename T> struct Pass<0, S, TPF, T> {
-    __device__ __forceinline__ static void run(const float *roi, int s, int q, T, const T (&te)[5], const T (&dt)[5],
+    __device__ __forceinline__ static void run(const float *roi, int s, int q, bool fused, T, const T (&te)[5],
+                                               const T (&dt)[5],
                                                T (&acc)[14], T (&vv)[5], T &chi2, T &dchi, T &dqmax)
     {
-        pass_sym<S, TPF, T>(roi, 1, s, q, te, dt, acc, vv, chi2, dchi, dqmax);
+        pass_sym<S, TPF, T>(roi, 1, s, q, fused, te, dt, acc, vv, chi2, dchi, dqmax);
     }
 };
 template <int S, int TPF, typename T> struct Pass<1, S, TPF, T> {
-    __device__ __forceinline__ static void run(const float *roi, int s, int q, T w0, const T (&te)[4],
+    __device__ __forceinline__ static void run(const float *roi, int s, int q, bool fused, T w0, const T (&te)[4],
                                                const T (&dt)[4], T (&acc)[9], T (&vv)[4], T &chi2, T &dchi,
                                                T &dqmax)
     {
-        pass_fixed<S, TPF, T>(roi, 1, s, q, w0, te, dt, acc, vv, chi2, dchi, dqmax);
+        pass_fixed<S, TPF, T>(roi, 1, s, q, fused, w0, te, dt, acc, vv, chi2, dchi, dqmax);
     }
 };
 template <int S, int TPF, typename T> struct Pass<7, S, TPF, T> {
-    __device__ __forceinline__ static void run(const float *roi, int s, int q, T, const T (&te)[7], const T (&dt)[7],
+    __device__ __forceinline__ static void run(const float *roi, int s, int q, bool, T, const T (&te)[7],
+                                               const T (&dt)[7],
                                                T (&acc)[27], T (&vv)[7], T &chi2, T &dchi, T &dqmax)
     {
         pass_ell<S, TPF, T>(roi, 1, s, q, te, dt, acc, vv, chi2, dchi, dqmax);
@@ -767,8 +769,8 @@ __device__ __forceinline__ void run_class(const K1Args &a, int r_class, int smem
             T vr[P];
 #pragma unroll
             for (int k = 0; k < P; ++k) vr[k] = v[k];
-            lmpar_scaled<P, T, ESC, kSmemState>(Ms, vr, invD, TPF == 1 || by_list ? sym_fuse(s, TPF) : 0, delta, par, z, a.pivot_thr, nl,
-                                    ne, sing, npiv, margin_fit, sstate ? sstate + 2 * NT + 4 * P : nullptr);
+            lmpar_scaled<P, T, ESC, kSmemState>(Ms, vr, invD, sym_fuse<ESC>(s, TPF), delta, par, z, a.pivot_thr, nl, ne, sing,
+                                    npiv, margin_fit, sstate ? sstate + 2 * NT + 4 * P : nullptr);
             if (leader) {
                 st[ST_LAMBDA] += nl;
                 st[ST_ESC] += ne;
@@ -778,12 +780,12 @@ __device__ __forceinline__ void run_class(const K1Args &a, int r_class, int smem
             if (sing) {
                 finish(T_SINGULAR);
             } else {
-                T pn2 = T(0);
+                T pn2 = T(0), z0;
 #pragma unroll
                 for (int k = 0; k < P; ++k) {
                     dx[k] = -z[k] * invD[k];
                     te[k] = th[k] + dx[k];
-                    pn2 += z[k] * z[k];
+                    add_square<T>(z[k], k, z0, pn2);
                 }
                 pnorm = fsqrt(pn2);
                 if (it_state == 1 && pnorm < delta) delta = pnorm;
@@ -792,8 +794,8 @@ __device__ __forceinline__ void run_class(const K1Args &a, int r_class, int smem
                 for (int i = 0; i < P; ++i) {
                     T row = T(0);
 #pragma unroll
-                    for (int j = 0; j < P; ++j) row += Ms[i <= j ? pku(P, i, j) : pku(P, j, i)] * z[j];
-                    qf += z[i] * row;
+                    for (int j = 0; j < P; ++j) row = fma(Ms[i <= j ? pku(P, i, j) : pku(P, j, i)], z[j], row);
+                    qf = fma(z[i], row, qf);
                 }
                 jdx2 = qf;
                 const bool bad = (METHOD == 0 && te[1] == T(0)) || (METHOD == 7 && (te[1] == T(0) || te[2] == T(0)));
@@ -816,7 +818,7 @@ __device__ __forceinline__ void run_class(const K1Args &a, int r_class, int smem
                 dt[k] = phase == 2 ? dx[k] : T(0);
                 tev[k] = te[k];
             }
-            Pass<METHOD, S, TPF, T>::run(myroi, s, q, w0, tev, dt, acc, vv, chi2, dchi, dqmax);
+            Pass<METHOD, S, TPF, T>::run(myroi, s, q, row_fused<METHOD, T, ESC>(s, TPF), w0, tev, dt, acc, vv, chi2, dchi, dqmax);
             if constexpr (TPF > 1 && sizeof(T) == 4) {
                 if (a.compensated) {
 #pragma unroll
@@ -866,13 +868,13 @@ __device__ __forceinline__ void run_class(const K1Args &a, int r_class, int smem
 #pragma unroll
                 for (int k = 0; k < P; ++k) v[k] = vv[k] * inv_s2;
                 fnorm = fn1;
-                T xn2 = T(0);
+                T xn2 = T(0), t0;
 #pragma unroll
                 for (int k = 0; k < P; ++k) {
                     const T cn = sqrt(A[pku(P, k, k)]);
                     D[k] = cn == T(0) ? T(1) : cn;
                     const T t = D[k] * theta_abs(k, th);
-                    xn2 += t * t;
+                    add_square<T>(t, k, t0, xn2);
                     dx[k] = T(0);
                 }
                 xnorm = sqrt(xn2);
@@ -912,12 +914,12 @@ __device__ __forceinline__ void run_class(const K1Args &a, int r_class, int smem
                     par /= temp;
                 }
                 if (ratio >= T(1e-4)) {
-                    T xn2 = T(0);
+                    T xn2 = T(0), t0;
 #pragma unroll
                     for (int k = 0; k < P; ++k) {
                         th[k] = te[k];
                         const T t = D[k] * theta_abs(k, th);
-                        xn2 += t * t;
+                        add_square<T>(t, k, t0, xn2);
                         v[k] = vv[k] * inv_s2;
                     }
 #pragma unroll

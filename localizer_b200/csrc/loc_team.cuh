@@ -116,16 +116,15 @@ template <int METHOD> __device__ __forceinline__ int team_unit(int u)
 }
 
 // One pixel's columns at the evaluation point; the expressions are those of
-// pass_sym, pass_fixed and pass_ell, statement for statement (krow in the
-// rounding that their row loops give it, see row_fuse_square).
+// pass_sym, pass_fixed and pass_ell, statement for statement.
 template <int METHOD, typename T> struct PixelEval;
 
 template <typename T> struct PixelEval<0, T> {
-    T A, x0, y0, b, dA, dxs, dys, db, A0, c1, ka_x, ka_r, cc, dc, m2dx, ra, rc;
-    bool sq;
-    __device__ __forceinline__ void prep(const T (&th)[5], const T (&dth)[5], T, int, bool square)
+    T A, x0, y0, b, dA, dxs, dys, db, A0, c1, ka_x, ka_r, cc, dc, m2dx;
+    bool fused;
+    __device__ __forceinline__ void prep(const T (&th)[5], const T (&dth)[5], T, int, bool row_fused)
     {
-        sq = square;
+        fused = row_fused;
         const T w = th[1], dw = dth[1];
         A = th[0];
         x0 = th[2];
@@ -145,15 +144,12 @@ template <typename T> struct PixelEval<0, T> {
         const T cpr = T(0.5) * w2i;
         dc = -T(2) * dw * (T(2) * w0c + dw) * cc * cpr;
         m2dx = -T(2) * dxs;
-        ra = sq ? -dxs : -dys;
-        rc = -mul_rn(dxs, dxs);
     }
     __device__ __forceinline__ T eval(int i, int j, T dat, T (&o)[8]) const
     {
         const T wy = (T)j - y0;
         const T wy2 = wy * wy;
-        const T t2 = fma(T(2), wy, dys);
-        const T krow = fma(ra, sq ? dxs : t2, sq ? -mul_rn(dys, t2) : rc);
+        const T krow = row_term<T>(fused, dxs, dys, wy);
         const T u = (T)i - x0;
         const T d2 = fma(u, u, wy2);
         const T e = Expo<T>::ex(d2 * c1);
@@ -177,11 +173,11 @@ template <typename T> struct PixelEval<0, T> {
 };
 
 template <typename T> struct PixelEval<1, T> {
-    T A, x0, y0, b, dA, dxs, dys, db, A0, c1, ka_x, cc, m2dx, ra, rc;
-    bool sq;
-    __device__ __forceinline__ void prep(const T (&th)[4], const T (&dth)[4], T w0, int, bool square)
+    T A, x0, y0, b, dA, dxs, dys, db, A0, c1, ka_x, cc, m2dx;
+    bool fused;
+    __device__ __forceinline__ void prep(const T (&th)[4], const T (&dth)[4], T w0, int, bool row_fused)
     {
-        sq = square;
+        fused = row_fused;
         A = th[0];
         x0 = th[1];
         y0 = th[2];
@@ -196,15 +192,12 @@ template <typename T> struct PixelEval<1, T> {
         ka_x = A * w2i;
         cc = T(0.5) * w2i;
         m2dx = -T(2) * dxs;
-        ra = sq ? -dxs : -dys;
-        rc = -mul_rn(dxs, dxs);
     }
     __device__ __forceinline__ T eval(int i, int j, T dat, T (&o)[8]) const
     {
         const T wy = (T)j - y0;
         const T wy2 = wy * wy;
-        const T t2 = fma(T(2), wy, dys);
-        const T krow = fma(ra, sq ? dxs : t2, sq ? -mul_rn(dys, t2) : rc);
+        const T krow = row_term<T>(fused, dxs, dys, wy);
         const T u = (T)i - x0;
         const T d2 = fma(u, u, wy2);
         const T e = Expo<T>::ex(d2 * c1);
@@ -354,13 +347,13 @@ template <int METHOD, typename T, int W>
 __device__ __forceinline__ bool team_pass(const float *roi, int s, T *chunk, T *sums, T *res,
                                        const T (&te)[Traits<METHOD>::P], const T (&dt)[Traits<METHOD>::P],
                                        const int (&entry)[TeamDims<METHOD>::NE / (32 * W) + 1], long long unit, T w0, T inv_s2,
-                                       int q_n, int wide, int tl)
+                                       int q_n, bool fused, int wide, int tl)
 {
     using D = TeamDims<METHOD>;
     using V2 = typename Vec2<T>::type;
     constexpr int NV = 2 * (D::PAIRS + 1);
     PixelEval<METHOD, T> px;
-    px.prep(te, dt, w0, threadIdx.x & 31, row_fuse_square<T>(s, q_n));
+    px.prep(te, dt, w0, threadIdx.x & 31, fused);
     // columns per partial sum; the first `more` have one more
     const int qmask = q_n - 1, qshift = q_n == 8 ? 3 : q_n >> 1;
     const int units = D::NB * q_n, per = s >> qshift, more = s & qmask;
@@ -648,7 +641,7 @@ __device__ __forceinline__ void team_fits(const TeamArgs &a, int r_cap, int n_al
                 bool sing = false;
                 unsigned nl = 0, ne = 0;
                 T npiv;
-                lmpar_scaled<P, T, ESC, false>(Ms, gv, inv_dv, sym_fuse(s, q_n), delta, par, z, ka.pivot_thr, nl, ne, sing,
+                lmpar_scaled<P, T, ESC, false>(Ms, gv, inv_dv, sym_fuse<ESC>(s, q_n), delta, par, z, ka.pivot_thr, nl, ne, sing,
                                                npiv, margin_fit);
                 if (tl == 0) {
                     st[ST_LAMBDA] += nl;
@@ -660,19 +653,19 @@ __device__ __forceinline__ void team_fits(const TeamArgs &a, int r_cap, int n_al
                     done = T_SINGULAR;
                     break;
                 }
-                T zk = z[0], pn2 = T(0), row = T(0);
+                T zk = z[0], pn2 = T(0), row = T(0), z0;
 #pragma unroll
                 for (int k = 0; k < P; ++k) {
                     if (k == lane) zk = z[k];
-                    pn2 += z[k] * z[k];
+                    add_square<T>(z[k], k, z0, pn2);
                 }
 #pragma unroll
                 for (int j = 0; j < P; ++j) {
                     const int lo = min(own, j), hi = max(own, j);
-                    row += Ms[pku(P, lo, hi)] * z[j];
+                    row = fma(Ms[pku(P, lo, hi)], z[j], row);
                 }
 #pragma unroll
-                for (int i = 0; i < P; ++i) jdx2 += z[i] * __shfl_sync(kFull, row, i);
+                for (int i = 0; i < P; ++i) jdx2 = fma(z[i], __shfl_sync(kFull, row, i), jdx2);
                 if (mine) {
                     dx = -zk * inv_d;
                     te = th + dx;
@@ -700,7 +693,7 @@ __device__ __forceinline__ void team_fits(const TeamArgs &a, int r_cap, int n_al
                 dtv[k] = s_dt[k];
             }
             const bool near = team_pass<METHOD, T, W>(roi, s, chunk, sums, alt, tev, dtv, entry, unit, w0, inv_s2, q_n,
-                                                      ka.compensated, tl);
+                                                      row_fused<METHOD, T, ESC>(s, q_n), ka.compensated, tl);
             if (tl == 0) {
                 if (first) {
                     st[ST_J] += 1;
@@ -755,12 +748,9 @@ __device__ __forceinline__ void team_fits(const TeamArgs &a, int r_cap, int n_al
                 th = te;
                 // |D x|, summed over the parameters in order
                 const T tx = sc * theta_abs(th);
-                T xn2 = T(0);
+                T xn2 = T(0), t0;
 #pragma unroll
-                for (int k = 0; k < P; ++k) {
-                    const T v = __shfl_sync(kFull, tx, k);
-                    xn2 = fma(v, v, xn2);
-                }
+                for (int k = 0; k < P; ++k) add_square<T>(__shfl_sync(kFull, tx, k), k, t0, xn2);
                 xnorm = sqrt(xn2);
                 fnorm = fn1;
                 T *x = cur;            // the trial point's sums become the current ones
