@@ -15,6 +15,7 @@
 // <= 0, centre outside the ROI, centre moved by more than 2 w0, integral
 // outside [1/2, 3/2] of the start, width outside [1/2, 3/2] w0.
 #include "../../include/localizer_b200.h"
+#include "loc_div.h"
 #include "loc_fit.cuh"
 
 #include <cuda_runtime.h>
@@ -67,27 +68,13 @@ struct RoiView {
     double xoff, yoff;
 };
 
-// a / b rounded correctly, with inv = RN(1 / b): Markstein's two residual
-// corrections ("Computation of elementary functions on the IBM RISC
-// System/6000 processor", IBM J. Res. Dev. 34, 1990). The first brings the
-// quotient within one ulp, the second rounds it correctly; both residuals
-// are exact while no intermediate leaves the normal range, which the caller
-// ensures (in_range).
-__device__ __forceinline__ double div_by(double a, double b, double inv)
-{
-    double q = a * inv;
-    q = __fma_rn(__fma_rn(-b, q, a), inv, q);
-    return __fma_rn(__fma_rn(-b, q, a), inv, q);
-}
-__device__ __forceinline__ bool in_range(double a) { return fabs(a) > 0x1p-300 && fabs(a) < 0x1p300; }
-
 // the negative log-likelihood at (x0, y0, sd, bg, nph), the same on every lane
 __device__ __forceinline__ double objective(double x0, double y0, double sd, double bg, double nph,
                                             const RoiView &roi, int lane)
 {
     const double norm = nph / (2 * kPi * sd * sd);
     const double inv = 1.0 / sd;
-    const bool fast = fabs(sd) > 0x1p-100 && fabs(sd) < 0x1p100;
+    const bool fast = div_fast(sd);
     double sum = 0.0;
     // this lane's pixel in the frame, kept in FP64 (small integers: exact)
     const int j0 = lane / roi.s;
@@ -500,7 +487,7 @@ cudaError_t enqueue_mlewg(const FitParams &p, unsigned long long *stats, cudaStr
              p.max_half_width > 0 ? (p.max_half_width < kMaxHalfWidth ? p.max_half_width : kMaxHalfWidth)
                                   : kMaxHalfWidth,
              p.out, p.flags, p.params_out, stats};
-    // a block's fits at the largest ROI the call admits: 75 KB at half-width 16
+    // a block's fits at the largest ROI the call admits: 45 KB at half-width 16
     const int smem = kWarps * smem_per_fit(a.r_cap);
     const cudaError_t e =
         cudaFuncSetAttribute(k_mlewg, cudaFuncAttributeMaxDynamicSharedMemorySize, kWarps * smem_per_fit(kMaxHalfWidth));
