@@ -74,7 +74,7 @@ XCOL = {0: 3, 1: 2, 5: 4, 7: 4}
 # DRAM bytes per fit of the whole plain-arm solver chain (every kernel of the
 # step) from an ncu capture, or None while no capture of the current kernels
 # exists
-TRAFFIC_PER_FIT = {"bytes": 1925.0, "source": "profiles/launches_dense500_plain.md (dense workload, 500 frames)"}
+TRAFFIC_PER_FIT = {"bytes": 1970.0, "source": "profiles/launches_dense500.md (dense workload, 500 frames)"}
 
 # the two reference builds: strict FP64 (the yardstick) and the reference's
 # own release flags (LinuxCompile.sh), which time the CPU baseline

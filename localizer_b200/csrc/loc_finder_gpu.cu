@@ -93,8 +93,9 @@ __device__ __forceinline__ void add_total(unsigned s, unsigned long long *total)
 // FP32 offsets from a pixel value c of the tile (exact integers), each lane
 // owns PX neighbouring columns and marches down the rows: the separable part
 // of the window is a 7-tap row sum and a 7-tap column sum over a register
-// ring, the sums of v and v^2 likewise, about 50 instructions a pixel (the
-// whole search of those frames: 15.2 -> 0.80 ms).
+// ring, the sums of v and v^2 likewise, with the tile's load and halo about
+// 105 instructions a pixel (counted; the whole search of those frames: 15.2 ->
+// 0.80 ms).
 //
 // With S = sum (v - c)^2, null = S - (sum (v - c))^2 / n and u = 2^-24, the
 // FP32 errors are |d conv| <= (2 ws + 2) u |gg| sqrt(S) + 2 u mean sqrt(n S)

@@ -1351,11 +1351,13 @@ cudaError_t launch_list_m(int m, const K1Args &ka, int r_cap, int tpb, int bps_r
 // Calls of at most this many candidates run on the team solver alone: that is
 // two fits for every warp of a full device (148 SMs x 12 warps). With one
 // thread per fit such a call leaves most of the device idle for as long as its
-// longest fit takes (160 symmetric fits 530 us, by teams 300 us).
+// longest fit takes (a call of 160 symmetric fits, FP64 re-run included, both
+// timed in turn: 437 us with a thread per fit, 235 us by teams). Like the lines
+// below it is written for the 148 SMs of a B200.
 constexpr int kTeamOnlyFits = 3552;
-// Lists of at most this many fits go to the teams at once (FP32, FP64). FP32:
-// any value from 300 to 3552 measures the same; FP64: 3552 is the best of 1 to
-// 3552 at 20 000 to 520 000 fits a call.
+// Lists of at most this many fits go to the teams at once (FP32, FP64). FP64:
+// 3552 is the best of 1 to 3552 at 20 000 to 520 000 fits a call. For FP32 the
+// line is not sensitive: 300 to 3552 measure the same, and it is the same one.
 constexpr int kTeamFits32 = 3552, kTeamFits64 = 3552;
 // A warp that has run dry hands its last fits over at this many groups or
 // fewer: FP32 with one thread per fit (the ellipsoidal models, whose fits
@@ -1374,10 +1376,10 @@ constexpr int kTeamFitsTiny = 300;
 // Lists of up to this many fits are solved by teams of four warps, longer ones
 // by teams of one. Four warps take 0.6 of the time per fit and the instructions
 // of nearly four, so they win while the longest fit sets the time: two (FP32)
-// and three (FP64) fits per resident block. Measured, one warp -> four: a frame
-// of 80 ellipsoidal fits 298 -> 248 us, 160 symmetric fits 362 -> 350 us, the
-// FP64 re-run of 262 of 520 000 symmetric fits 6.30 -> 5.70 ms for the call; with
-// 2 400 ellipsoidal re-runs 10.6 -> 11.8 ms, so they keep one warp.
+// and three (FP64) fits per resident block. Measured, one warp -> four: the
+// solver's part of a frame of 80 ellipsoidal fits 298 -> 248 us, the FP64 re-run
+// of 262 of 520 000 symmetric fits 6.30 -> 5.70 ms for the call; with 2 400
+// ellipsoidal re-runs 10.6 -> 11.8 ms, so they keep one warp.
 constexpr int kBlockFits32 = 1184, kBlockFits64 = 1332;
 
 template <int METHOD, typename T, bool ESC>

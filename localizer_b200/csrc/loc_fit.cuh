@@ -19,13 +19,14 @@ struct Scratch {
     int *meta;           // kMetaInts: class table (see loc_fit.cu)
     void *state;         // n * state_stride(method) elements of the solver precision
     unsigned long long *stats;  // 8 counters
-    int *cont;           // n: continuation queue (fits suspended after the level-0 budget)
+    int *cont;           // n: fits past the level-0 budget from the front, fits left to the teams from the back
     float *cont_state;   // n * cont stride: their saved solver state
-    int *cls2;           // n: half-width class of fits re-run in FP64, -1 otherwise
-    int *order2;         // n: their queue (fits whose FP32 solve ended within the level-0 budget)
-    int *meta2;          // kMetaInts: its class table
-    int *order3;         // n: queue of the long re-runs (FP32 solve outlived the level-0 budget)
-    int *meta3;          // kMetaInts: its class table
+    int *cls2;           // n: half-width class of fits re-run in FP64, -1 otherwise (-2: suspended)
+    int *order2;         // n: lists of the short re-runs, of first-level fits from the front, of suspended ones
+                         // from the back
+    int *meta2;          // kMetaInts: their lengths and cursors
+    int *order3;         // n: lists of the long re-runs (more FP32 iterations than long_rerun_iters), the same
+    int *meta3;          // kMetaInts: their lengths and cursors
     double *state64;     // n * state_stride(method): FP64 state of re-run fits
     float *init;         // n * P: proposed starts (warm mode only)
 };
